@@ -92,10 +92,10 @@ typedef struct QfTensorDesc {
     float* v_scale;       /* BLOCK: [ceil(numel/128)]; RANK1: row maxima [rows]; in/out          */
     float* v_col;         /* RANK1: column maxima [cols]; in/out                                 */
     float* v_row_new;     /* RANK1: scratch for the new row maxima: [2*rows] if v_row_rcp is null
-                             (maxima, then their reciprocals), else [rows]                         */
+                             (new maxima, then a copy of the old ones), else [rows]                */
     float* v_col_new;     /* RANK1: the same for the columns: [2*cols], or [cols] with v_col_rcp  */
-    float* v_row_rcp;     /* RANK1, optional: separate scratch [rows] for the reciprocals          */
-    float* v_col_rcp;     /* RANK1, optional: separate scratch [cols] for the reciprocals          */
+    float* v_row_rcp;     /* RANK1, optional: separate scratch [rows] for the second half          */
+    float* v_col_rcp;     /* RANK1, optional: separate scratch [cols] for the second half          */
     int64_t numel;        /* elements this record covers                                         */
     int64_t rows;         /* RANK1 only; rows * cols == numel unless the record is partial       */
     int64_t cols;
@@ -126,9 +126,9 @@ size_t qf_workspace_bytes(int n_tensors);
  * cuda_adamw_kernels.cu:136-164, :422-469; driver loop optim/fused_quantfour.py:171-292).
  *
  * `descs` and `hypers` are host arrays.  For RANK1 tensors the call (1) clears v_row_new/v_col_new,
- * (2) accumulates the new maxima, (3) stores their reciprocals in the second halves of the scratch
- * arrays, updates and requantizes using the old maxima for dequantize and the new ones for quantize,
- * (4) copies the new maxima into v_scale/v_col.
+ * (2) accumulates the new maxima, (3) copies the old maxima into the second halves of the scratch
+ * arrays, updates and requantizes using that copy for dequantize and the new maxima for quantize, and
+ * (4) stores the new maxima into v_scale/v_col.
  */
 int qf_step_multi(const QfTensorDesc* descs, int n_tensors, const QfHyper* hypers, int n_hypers,
                   void* workspace, size_t workspace_bytes, int device, void* stream);
@@ -310,7 +310,7 @@ int qf_dequantize_rank1(const uint8_t* codes, const float* row_max, const float*
  * allocation at that point would either fail or stall the device (device allocations synchronise);
  * plug-in hosts that only pass tensors through and own no allocator are in the same position.  For them
  * the scratch qf_step_multi asks for (descriptor table, status word, new row / column maxima and their
- * reciprocals) lives inside the library, in a device array of QF_NOALLOC_MAX_ROWS_PLUS_COLS * 8 + 1024
+ * a copy of the old ones) lives inside the library, in a device array of QF_NOALLOC_MAX_ROWS_PLUS_COLS * 8 + 1024
  * bytes (about 1 MiB) that every GPU which loads the library holds until the process ends.
  *
  * Limits and rules:

@@ -38,13 +38,15 @@ int fail(int code, const char* fmt, ...) {
 
 constexpr size_t kStatusBytes = 256;  // head of the workspace: status word, then padding
 
-constexpr int kTables = 4;  // prefix sums: main/panel, main/flat, pre/panel, pre/flat
+constexpr int kTables = 5;  // prefix sums: main/panel, main/flat, pre/panel, pre/flat, row and column maxima
 size_t table_bytes(int n) { return static_cast<size_t>(n) * sizeof(qf::DevTensor) + kTables * (static_cast<size_t>(n) + 1) * 8; }
 size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 bool valid_dtype(int dtype) { return dtype == QF_F32 || dtype == QF_BF16 || dtype == QF_F16; }
 size_t elem_size(int dtype) { return dtype == QF_F32 ? 4 : 2; }
+
+int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 int64_t flat_items(int64_t numel) {
     const int64_t per = static_cast<int64_t>(qf::kPanelCols) * qf::kRowsPerItem;
@@ -91,27 +93,34 @@ bool drop_cache_entry(WsCache& c, bool wait) {
     return true;
 }
 
-enum { kMainPanel = 0, kMainFlat = 1, kPrePanel = 2, kPreFlat = 3 };
+enum { kMainPanel = 0, kMainFlat = 1, kPrePanel = 2, kPreFlat = 3, kRoll = 4 };
 struct Plan {
     int n = 0;                    // tensors in the table (zero-size tensors dropped)
-    int64_t items[kTables] = {0, 0, 0, 0};
+    int64_t items[kTables] = {};
     int n_rank1 = 0;
     bool any_f32_panel = false;   // sizes the staging ring of the panel kernel
     bool any_bf16_panel = false;
+    bool any_f16_panel = false;
     qf::DevTensor* d_tensors = nullptr;
-    int64_t* d_base[kTables] = {nullptr, nullptr, nullptr, nullptr};
+    int64_t* d_base[kTables] = {};
     uint32_t* d_status = nullptr;
 };
 
-// Rows per item of the second pass over rank-1 panels: the longest of 64 / 32 / 16 that still gives every warp slot
-// of the device (two CTAs of eight warps per SM) an item; `bands64` = sum over the panel tensors of rows * panels / 64.
 int sm_count();
-int main_rows_for(int64_t items64) {
-    const int64_t slots = static_cast<int64_t>(sm_count()) * qf::kMainMinCtas * qf::kWarpsPerCta;
-    int rows = qf::kMainRowsPerItem;
-    while (rows > 16 && items64 * (qf::kMainRowsPerItem / rows) < slots) rows /= 2;
-    return rows;
+// Length of a work item (rows of a panel, runs of the flat mapping): the longest of longest, longest / 2, .. shortest
+// that still gives every slot of the device (`per_sm` per SM) one; `items` = the number of items of the longest form.
+int item_length(int64_t items, int longest, int shortest, int per_sm) {
+    const int64_t slots = static_cast<int64_t>(sm_count()) * per_sm;
+    int len = longest;
+    while (len > shortest && items * (longest / len) < slots) len /= 2;
+    return len;
 }
+int main_rows_for(int64_t items) {
+    return item_length(items, qf::kMainRowsPerItem, qf::kMinMainRowsPerItem, qf::kMainMinCtas * qf::kWarpsPerCta);
+}
+// two CTA items per slot: 512 rows per item left the device a ragged last wave (202 M elements: 139 -> 125 us)
+int pre_rows_for(int64_t items) { return item_length(items, qf::kPreRowsPerItem, qf::kMinPreRowsPerItem, 2 * qf::kPreMinCtas); }
+int flat_runs_for(int64_t items) { return item_length(items, qf::kRowsPerItem, qf::kMinRowsPerItem, qf::kMainMinCtas * qf::kWarpsPerCta); }
 
 int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* workspace, size_t workspace_bytes,
                int device, cudaStream_t stream, Plan* plan, bool upload = true) {
@@ -174,21 +183,21 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
             t.vcol = d.v_col;
             t.vrow_new = d.v_row_new;
             t.vcol_new = d.v_col_new;
-            t.vrow_rcp = d.v_row_rcp ? d.v_row_rcp : d.v_row_new + d.rows;
-            t.vcol_rcp = d.v_col_rcp ? d.v_col_rcp : d.v_col_new + d.cols;
+            t.vrow_old = d.v_row_rcp ? d.v_row_rcp : d.v_row_new + d.rows;
+            t.vcol_old = d.v_col_rcp ? d.v_col_rcp : d.v_col_new + d.cols;
             t.flat_off = d.flat_offset;
-            if (!aligned(t.vrow_rcp, 4) || !aligned(t.vcol_rcp, 4)) return fail(QF_ERR_BAD_ARG, "tensor %d: rank-1 buffers misaligned", i);
+            if (!aligned(t.vrow_old, 4) || !aligned(t.vcol_old, 4)) return fail(QF_ERR_BAD_ARG, "tensor %d: rank-1 buffers misaligned", i);
             const bool whole = d.flat_offset == 0 && d.rows * d.cols == d.numel;
-            const bool panel = whole && d.dtype != QF_F16 && d.numel < (1ll << 31) && vec && d.cols % qf::kPanelCols == 0 && aligned(d.v_col, 16) && aligned(d.v_col_new, 16) &&
-                               aligned(t.vcol_rcp, 16);
+            const bool panel = whole && d.numel < (1ll << 31) && vec && d.cols % qf::kPanelCols == 0 && aligned(d.v_col, 16) && aligned(d.v_col_new, 16) &&
+                               aligned(t.vcol_old, 16);
             if (panel) {
                 t.flags |= qf::kFlagPanel;
                 t.panels = static_cast<int32_t>(d.cols / qf::kPanelCols);
-                t.main_rows = qf::kMainRowsPerItem;
                 items = (d.rows + qf::kMainRowsPerItem - 1) / qf::kMainRowsPerItem * t.panels;
-                pre_items = (d.rows + qf::kPreRowsPerItem - 1) / qf::kPreRowsPerItem * t.panels;
+                pre_items = ceil_div(d.rows, qf::kPreRowsPerItem * qf::kWarpsPerCta) * t.panels;
                 if (d.dtype == QF_F32) plan->any_f32_panel = true;
                 if (d.dtype == QF_BF16) plan->any_bf16_panel = true;
+                if (d.dtype == QF_F16) plan->any_f16_panel = true;
             }
             ++n_rank1;
         }
@@ -198,20 +207,28 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
         base[kMainFlat].push_back(base[kMainFlat].back() + (panel ? 0 : items));
         base[kPrePanel].push_back(base[kPrePanel].back() + (rank1 && panel ? pre_items : 0));
         base[kPreFlat].push_back(base[kPreFlat].back() + (rank1 && !panel ? pre_items : 0));
+        base[kRoll].push_back(base[kRoll].back() + (rank1 ? ceil_div(d.rows + d.cols, qf::kRollEntries) : 0));
         tab.push_back(t);
     }
     const int n = static_cast<int>(tab.size());
-    // a small launch: shorter items in the second pass, so that the whole device takes part
-    const int main_rows = main_rows_for(base[kMainPanel].back());
-    if (main_rows != qf::kMainRowsPerItem) {
-        int64_t acc = 0;
-        for (int i = 0; i < n; ++i) {
-            if (tab[i].flags & qf::kFlagPanel) {
-                tab[i].main_rows = main_rows;
-                acc += (static_cast<int64_t>(tab[i].rows) + main_rows - 1) / main_rows * tab[i].panels;
-            }
-            base[kMainPanel][i + 1] = acc;
+    // a small launch: shorter items, so that the whole device takes part
+    const int main_rows = main_rows_for(base[kMainPanel].back()), pre_rows = pre_rows_for(base[kPrePanel].back());
+    const int flat_runs = flat_runs_for(base[kMainFlat].back());
+    int64_t acc[kTables] = {};
+    for (int i = 0; i < n; ++i) {
+        qf::DevTensor& t = tab[i];
+        t.main_rows = main_rows;
+        t.pre_rows = pre_rows;
+        t.flat_runs = flat_runs;
+        if (t.flags & qf::kFlagPanel) {
+            acc[kMainPanel] += ceil_div(t.rows, main_rows) * t.panels;
+            acc[kPrePanel] += ceil_div(t.rows, pre_rows * qf::kWarpsPerCta) * t.panels;
+        } else {
+            const int64_t items = ceil_div(t.numel, static_cast<int64_t>(qf::kPanelCols) * flat_runs);
+            acc[kMainFlat] += items;
+            if (t.kind == QF_KIND_RANK1) acc[kPreFlat] += items;
         }
+        for (int k = 0; k < kRoll; ++k) base[k][i + 1] = acc[k];
     }
     plan->n = n;
     plan->n_rank1 = n_rank1;
@@ -281,7 +298,7 @@ unsigned persistent_grid(int64_t items, int per_sm, int waves = kGridWaves) {
 }
 
 void roll(const Plan& pl, int mode, cudaStream_t stream) {
-    qf::rank1_roll_kernel<<<pl.n * qf::kRollSlices, qf::kThreads, 0, stream>>>(pl.d_tensors, pl.n, mode);
+    qf::rank1_roll_kernel<<<static_cast<unsigned>(pl.items[kRoll]), qf::kThreads, 0, stream>>>(pl.d_tensors, pl.d_base[kRoll], pl.n, mode);
 }
 
 qf::Sched no_sched() {
@@ -290,21 +307,26 @@ qf::Sched no_sched() {
     return sc;
 }
 
+unsigned panel_pre_grid(int64_t items) {   // one item per CTA and turn
+    return static_cast<unsigned>(std::min<int64_t>(items, static_cast<int64_t>(sm_count()) * qf::kPreMinCtas * kGridWaves));
+}
+
 template <bool SCALE, bool SCHED>
 int launch_pre_panel(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
     const int dyn = qf::pre_dyn_smem(pl.any_f32_panel);
     QF_CUDA(cudaFuncSetAttribute(qf::step_pre_kernel<true, SCALE, SCHED>, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::pre_dyn_smem(true)));
-    qf::step_pre_kernel<true, SCALE, SCHED><<<persistent_grid(pl.items[kPrePanel], qf::kPreMinCtas), qf::kThreads, dyn, stream>>>(
+    qf::step_pre_kernel<true, SCALE, SCHED><<<panel_pre_grid(pl.items[kPrePanel]), qf::kThreads, dyn, stream>>>(
         pl.d_tensors, pl.d_base[kPrePanel], pl.n, hp, dyn / qf::kWarpsPerCta, pl.d_status, sc);
     return QF_OK;
 }
 
 // `sched`: null, or the device-resident hyper-parameter table the kernels read instead of `hp`; `scaled` then says
 // whether some row of it carries a gradient scale (the host cannot look).
-int launch_pre(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStream_t stream, const qf::Sched* sched = nullptr,
+// `keep`: the second half follows in the same call; the copy of the old maxima it reads is then made here as well.
+int launch_pre(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStream_t stream, bool keep, const qf::Sched* sched = nullptr,
                bool scaled = false) {
     if (pl.n_rank1 == 0) return QF_OK;
-    roll(pl, qf::kRollClear, stream);
+    roll(pl, qf::kRollClear | (keep ? qf::kRollKeep : 0), stream);
     if (pl.items[kPrePanel]) {
         // the variant that rewrites the gradients runs only when some set asks for it
         if (!sched)
@@ -336,17 +358,23 @@ int launch_main_panel_dt(const Plan& pl, const qf::HyperPack& hp, const qf::Push
     QF_CUDA(cudaFuncSetAttribute(qf::step_main_kernel<true, PUSH, BC1, SCHED, RELAXED, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  qf::main_dyn_smem(true)));
     qf::step_main_kernel<true, PUSH, BC1, SCHED, RELAXED, DT><<<persistent_grid(pl.items[kMainPanel], qf::kMainMinCtas), qf::kThreads, dyn, stream>>>(
-        pl.d_tensors, pl.d_base[kMainPanel], pl.n, hp, ring, pl.d_status, pp, sc);
+        pl.d_tensors, pl.d_base[kMainPanel], pl.n, hp, ring, pl.d_status, pp, sc, pl.d_base[kRoll], static_cast<int>(pl.items[kRoll]));
     return QF_OK;
 }
 // A launch whose panel tensors are all of one dtype takes the kernel that carries that dtype's loop only (the plain
 // step, the common case; the rarer variants keep the two-dtype kernel): 1.4 % faster, measured.
 template <bool PUSH, bool BC1, bool SCHED, bool RELAXED = false>
 int launch_main_panel(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, cudaStream_t stream) {
-    if (!PUSH && !SCHED && !RELAXED && !pl.any_f32_panel) return launch_main_panel_dt<false, BC1, false, false, 1>(pl, hp, pp, sc, stream);
-    if (!PUSH && !SCHED && !RELAXED && !pl.any_bf16_panel) return launch_main_panel_dt<false, BC1, false, false, 2>(pl, hp, pp, sc, stream);
+    if (!PUSH && !SCHED && !RELAXED) {
+        if (!pl.any_f32_panel && !pl.any_f16_panel) return launch_main_panel_dt<false, BC1, false, false, 1>(pl, hp, pp, sc, stream);
+        if (!pl.any_bf16_panel && !pl.any_f16_panel) return launch_main_panel_dt<false, BC1, false, false, 2>(pl, hp, pp, sc, stream);
+        if (!pl.any_bf16_panel && !pl.any_f32_panel) return launch_main_panel_dt<false, BC1, false, false, 3>(pl, hp, pp, sc, stream);
+    }
     return launch_main_panel_dt<PUSH, BC1, SCHED, RELAXED, 0>(pl, hp, pp, sc, stream);
 }
+
+// The new maxima are stored by the panel launch where there is one, else by the flat one.
+int flat_rolls(const Plan& pl) { return pl.items[kMainPanel] ? 0 : static_cast<int>(pl.items[kRoll]); }
 
 // bc_one: every hyper-parameter set of the call has bc2s == 1 exactly (late in a run): the panel kernel then
 // runs the variant without the division by it.
@@ -366,17 +394,18 @@ int launch_main_kernels(const Plan& pl, const qf::HyperPack& hp, const qf::PushP
     }
     if (pl.items[kMainFlat])
         qf::step_main_kernel<false, PUSH><<<persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), qf::kThreads, 0, stream>>>(
-            pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, pp, no_sched());
+            pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, pp, no_sched(), pl.d_base[kRoll], flat_rolls(pl));
     return QF_OK;
 }
 
 // `push`: null, or the peer copies of the parameter buffer the kernels also store into.
 // `sched`: null, or the device-resident hyper-parameter table the kernels read instead of `hp` (no peer stores then,
 // and always the variant that divides by the bias correction: what the table holds is not known to the host).
-int launch_main(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStream_t stream, const qf::PushPack* push = nullptr,
+// `kept`: launch_pre of the same call has made the copy of the old maxima.
+int launch_main(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStream_t stream, bool kept, const qf::PushPack* push = nullptr,
                 const qf::Sched* sched = nullptr, bool relaxed = false) {
     if (pl.n == 0) return QF_OK;
-    if (pl.n_rank1) roll(pl, qf::kRollRecip, stream);
+    if (pl.n_rank1 && !kept) roll(pl, qf::kRollKeep, stream);
     bool bc_one = true;
     for (int k = 0; k < n_hypers; ++k) bc_one = bc_one && hp.h[k].fast && hp.h[k].h.bc2s == 1.0f;
     qf::PushPack none;
@@ -386,13 +415,12 @@ int launch_main(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStrea
             if (int rc = launch_main_panel<false, false, true>(pl, hp, none, *sched, stream)) return rc;
         if (pl.items[kMainFlat])
             qf::step_main_kernel<false, false, false, true><<<persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), qf::kThreads, 0, stream>>>(
-                pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, none, *sched);
+                pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, none, *sched, pl.d_base[kRoll], flat_rolls(pl));
     } else if (push && push->n > 0) {
         if (int rc = launch_main_kernels<true>(pl, hp, *push, bc_one, stream)) return rc;
     } else {
         if (int rc = launch_main_kernels<false>(pl, hp, none, bc_one, stream, relaxed)) return rc;
     }
-    if (pl.n_rank1) roll(pl, qf::kRollCommit, stream);
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -412,9 +440,9 @@ int step_common(const QfTensorDesc* descs, int n_tensors, const QfHyper* hypers,
     memset(&hp, 0, sizeof hp);
     for (int k = 0; k < n_hypers; ++k) hp.h[k] = widen_hyper(hypers[k]);
     if (pre)
-        if (int rc = launch_pre(pl, hp, n_hypers, st)) return rc;
+        if (int rc = launch_pre(pl, hp, n_hypers, st, main_)) return rc;
     if (main_)
-        if (int rc = launch_main(pl, hp, n_hypers, st, push, nullptr, relaxed)) return rc;
+        if (int rc = launch_main(pl, hp, n_hypers, st, pre, push, nullptr, relaxed)) return rc;
     return QF_OK;
 }
 
@@ -426,6 +454,11 @@ int check_1d(const void* a, const void* b, int64_t numel, const char* what) {
 
 unsigned flat_grid(int64_t numel) {
     return static_cast<unsigned>((flat_items(numel) + qf::kWarpsPerCta - 1) / qf::kWarpsPerCta);
+}
+
+// Grid of single_tensor_kernel: one item per warp.
+unsigned single_grid(const qf::DevTensor& t) {
+    return static_cast<unsigned>(ceil_div(t.numel, static_cast<int64_t>(qf::kPanelCols) * t.flat_runs * qf::kWarpsPerCta));
 }
 
 }  // namespace
@@ -496,8 +529,8 @@ int qf_step_scheduled(const QfTensorDesc* descs, int n_tensors, int n_hypers, vo
     sc.n_hypers = n_hypers;
     qf::HyperPack hp;
     memset(&hp, 0, sizeof hp);
-    if (int rc = launch_pre(pl, hp, 0, st, &sc, (flags & QF_SCHED_GRAD_SCALE) != 0)) return rc;
-    if (int rc = launch_main(pl, hp, 0, st, nullptr, &sc)) return rc;
+    if (int rc = launch_pre(pl, hp, 0, st, true, &sc, (flags & QF_SCHED_GRAD_SCALE) != 0)) return rc;
+    if (int rc = launch_main(pl, hp, 0, st, true, nullptr, &sc)) return rc;
     qf::sched_advance_kernel<<<1, 32, 0, st>>>(device_counters, schedule_rows, (flags & QF_SCHED_TAIL_REPEATS) != 0, pl.d_status);
     QF_CUDA(cudaGetLastError());
     return QF_OK;
@@ -706,12 +739,13 @@ int qf_fused_4bit(void* p, const void* g, void* exp, void* sq, float* exp_scale,
     t.vs = sq_scale;
     t.numel = numel;
     t.kind = QF_KIND_BLOCK;
+    t.flat_runs = flat_runs_for(flat_items(numel));
     t.dtype = dtype;
     if (aligned(p, 16) && aligned(g, 16) && aligned(exp, 4) && aligned(sq, 4)) t.flags |= qf::kFlagVec;
     QfHyper h;
     qf_make_hyper(lr, beta1, beta2, eps, weight_decay, step, &h);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    qf::single_tensor_kernel<<<flat_grid(numel), qf::kThreads, 0, st>>>(t, widen_hyper(h));
+    qf::single_tensor_kernel<<<single_grid(t), qf::kThreads, 0, st>>>(t, widen_hyper(h));
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -735,12 +769,13 @@ int qf_fused_single_tensor(void* p, const void* g, float* exp_avg, float* exp_av
     t.v = reinterpret_cast<char*>(exp_avg_sq);
     t.numel = numel;
     t.kind = QF_KIND_FP32;
+    t.flat_runs = flat_runs_for(flat_items(numel));
     t.dtype = dtype;
     if (aligned(p, 16) && aligned(g, 16) && aligned(exp_avg, 16) && aligned(exp_avg_sq, 16)) t.flags |= qf::kFlagVec;
     QfHyper h;
     qf_make_hyper(lr, beta1, beta2, eps, weight_decay, step, &h);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    qf::single_tensor_kernel<<<flat_grid(numel), qf::kThreads, 0, st>>>(t, widen_hyper(h));
+    qf::single_tensor_kernel<<<single_grid(t), qf::kThreads, 0, st>>>(t, widen_hyper(h));
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -835,9 +870,9 @@ int qf_dequantize_rank1(const uint8_t* codes, const float* row_max, const float*
 // ---- the step of one rank-1 tensor for callers that cannot allocate ------------------------------------
 //
 // Scratch of this entry point: a status word, the one-entry descriptor table and the new row / column
-// maxima with their reciprocals.  It lives in this translation unit as a device array; each GPU that loads
+// maxima with the copy of the old ones.  It lives in this translation unit as a device array; each GPU that loads
 // the library keeps its own copy of it for the life of the process.
-constexpr size_t kNoAllocHeader = 1024;  // status word, tensor record, four two-entry prefix tables
+constexpr size_t kNoAllocHeader = 1024;  // status word, tensor record, two-entry prefix tables
 constexpr size_t kNoAllocBytes = kNoAllocHeader + 8 * static_cast<size_t>(QF_NOALLOC_MAX_ROWS_PLUS_COLS);
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -880,7 +915,7 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     if (int rc = noalloc_scratch(device, &scratch)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    // layout: [status | tensor record | 4 prefix tables][row maxima, reciprocals][column maxima, reciprocals]
+    // layout: [status | tensor record | prefix tables][new row maxima, copy of the old ones][the same for the columns]
     float* row_new = reinterpret_cast<float*>(scratch + kNoAllocHeader);
     float* col_new = row_new + 2 * ((rows + 3) / 4 * 4);  // keeps the column part 16-byte aligned
     if (reinterpret_cast<unsigned char*>(col_new + 2 * cols) > scratch + kNoAllocBytes)
@@ -897,8 +932,8 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     t.vcol = v_col;
     t.vrow_new = row_new;
     t.vcol_new = col_new;
-    t.vrow_rcp = row_new + rows;
-    t.vcol_rcp = col_new + cols;
+    t.vrow_old = row_new + rows;
+    t.vcol_old = col_new + cols;
     t.numel = rows * cols;
     t.rows = static_cast<int32_t>(rows);
     t.cols = static_cast<int32_t>(cols);
@@ -906,13 +941,15 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     t.dtype = dtype;
     const bool vec = aligned(p, 16) && aligned(g, 16) && aligned(m_codes, 4) && aligned(v_codes, 4);
     if (vec) t.flags |= qf::kFlagVec;
-    int64_t items = flat_items(t.numel), pre_items = items;
-    if (vec && dtype != QF_F16 && t.numel < (1ll << 31) && cols % qf::kPanelCols == 0 && aligned(v_col, 16)) {
+    t.flat_runs = flat_runs_for(flat_items(t.numel));
+    int64_t items = ceil_div(t.numel, static_cast<int64_t>(qf::kPanelCols) * t.flat_runs), pre_items = items;
+    if (vec && t.numel < (1ll << 31) && cols % qf::kPanelCols == 0 && aligned(v_col, 16)) {
         t.flags |= qf::kFlagPanel;
         t.panels = static_cast<int32_t>(cols / qf::kPanelCols);
-        t.main_rows = main_rows_for((rows + qf::kMainRowsPerItem - 1) / qf::kMainRowsPerItem * t.panels);
-        items = (rows + t.main_rows - 1) / t.main_rows * t.panels;
-        pre_items = (rows + qf::kPreRowsPerItem - 1) / qf::kPreRowsPerItem * t.panels;
+        t.main_rows = main_rows_for(ceil_div(rows, qf::kMainRowsPerItem) * t.panels);
+        t.pre_rows = pre_rows_for(ceil_div(rows, qf::kPreRowsPerItem * qf::kWarpsPerCta) * t.panels);
+        items = ceil_div(rows, t.main_rows) * t.panels;
+        pre_items = ceil_div(rows, t.pre_rows * qf::kWarpsPerCta) * t.panels;
     }
     const bool panel = t.flags & qf::kFlagPanel;
 
@@ -928,6 +965,7 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     h.base[kMainFlat][1] = panel ? 0 : items;
     h.base[kPrePanel][1] = panel ? pre_items : 0;
     h.base[kPreFlat][1] = panel ? 0 : pre_items;
+    h.base[kRoll][1] = ceil_div(rows + cols, qf::kRollEntries);
     // The header goes up from this stack frame; a copy from pageable memory returns once the source has
     // been staged (for which the runtime may make the host wait for earlier work of the stream), so the frame
     // may die afterwards.  The status words ahead of the tensor record are not part of the copy: they
@@ -940,6 +978,7 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     pl.n_rank1 = 1;
     pl.any_f32_panel = panel && dtype == QF_F32;
     pl.any_bf16_panel = panel && dtype == QF_BF16;
+    pl.any_f16_panel = panel && dtype == QF_F16;
     pl.d_status = reinterpret_cast<uint32_t*>(scratch);
     pl.d_tensors = reinterpret_cast<qf::DevTensor*>(scratch + offsetof(Header, t));
     for (int k = 0; k < kTables; ++k) {
@@ -949,8 +988,8 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     qf::HyperPack hp;
     memset(&hp, 0, sizeof hp);
     hp.h[0] = widen_hyper(*hyper);
-    if (int rc = launch_pre(pl, hp, 1, st)) return rc;   // clears the new maxima first: the array keeps the last call's
-    return launch_main(pl, hp, 1, st);
+    if (int rc = launch_pre(pl, hp, 1, st, true)) return rc;   // clears the new maxima first: the array keeps the last call's
+    return launch_main(pl, hp, 1, st, true);
 }
 
 int qf_read_status_noalloc(int device, void* stream, uint32_t* status) {

@@ -25,13 +25,20 @@ namespace qf {
 constexpr int kWarpsPerCta = 8;
 constexpr int kThreads = kWarpsPerCta * 32;
 constexpr int kPanelCols = 256;   // columns one warp covers: 32 lanes x 8 elements = two 128-blocks
-constexpr int kRowsPerItem = 16;  // rows (of kPanelCols elements) one warp work item covers
-constexpr int kMainRowsPerItem = 64;  // rows of one item of the second pass over a rank-1 panel: longer items
-                                      // amortise the per-item set-up (column maxima into shared memory); a launch
-                                      // with too few such items to give every warp slot of the device one takes
-                                      // 32 or 16 rows per item instead (always an even number: rows go in pairs)
-constexpr int kPreRowsPerItem = 64;  // the same for the first pass over a rank-1 panel: each item ends with one
-                                     // red.max per column, so longer items mean fewer contended atomics
+// Longest work items.  A launch with too few items of that length to give every slot of the device one takes shorter
+// ones, halving down to the shortest (qf_api.cu, item_length): a warp that walks a long item alone is all latency
+// (one 4096-element vector as 16 runs of one warp: 22 us; as 16 items: 5 us).
+constexpr int kRowsPerItem = 16;      // flat mapping: runs of kPanelCols elements per warp
+constexpr int kMinRowsPerItem = 1;
+constexpr int kMainRowsPerItem = 64;  // second pass over a rank-1 panel, rows per warp (an even number mostly: rows go in
+                                      // pairs): longer items amortise the per-item set-up.  At most 32 / 16 measured +2.5 % /
+                                      // +9 % on the second pass over 645 M bf16 elements.
+constexpr int kMinMainRowsPerItem = 4;
+constexpr int kPreRowsPerItem = 64;   // first pass over a rank-1 panel, rows per warp of a CTA's item.  The CTA combines its
+                                      // warps' column maxima first, so an item ends with one red.max per column for eight
+                                      // times as many rows; below 16 rows the atomics on the column maxima show (12.6 M
+                                      // elements: 8 rows 22.9, 16 rows 19.0 us for the first half).
+constexpr int kMinPreRowsPerItem = 16;
 constexpr unsigned kFull = 0xffffffffu;
 
 // Code books.  Literals as in optim/cuda_adamw_kernels.cu:25-98 (= optim/adamw_fourbit_triton.py:16-97):
@@ -147,7 +154,7 @@ struct Elem<__nv_bfloat16> {
 };
 
 // fp16 parameters and gradients (the reference's launcher dispatches half as well, optim/cuda_adamw_kernels.cu:443):
-// widened exactly, rounded to nearest even on the way back.  Tensors of this dtype always take the flat mapping.
+// widened exactly, rounded to nearest even on the way back.
 template <>
 struct Elem<__half> {
     static __device__ __forceinline__ void load8(const char* base, int64_t e, float (&x)[8]) {

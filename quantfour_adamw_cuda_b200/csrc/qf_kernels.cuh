@@ -4,12 +4,12 @@
 // load of bf16 parameters, one 32-bit word of codes), so a warp covers 256 consecutive elements = two
 // 128-element quantization blocks, and a block's abs-max is a 4-step shuffle among 16 lanes with no
 // shared memory and no CTA barrier.  A warp work item is
-//   * for rank-1 tensors whose column count is a multiple of 256 ("panel" mapping): 64 rows of one
+//   * for rank-1 tensors whose column count is a multiple of 256 ("panel" mapping): up to 64 rows of one
 //     256-column panel.  A lane keeps the same 8 columns for the whole item, so everything that depends on
 //     the column only (old and new column maxima, their reciprocals) is fetched once per item (registers in
 //     the first pass, the warp's slice of shared memory in the main pass), and the first pass reduces column
-//     maxima over the rows in registers before touching global memory;
-//   * otherwise ("flat" mapping): kRowsPerItem (16) consecutive runs of 256 flattened elements.
+//     maxima over the rows in registers, then over the warps of the CTA, before touching global memory;
+//   * otherwise ("flat" mapping): up to kRowsPerItem (16) consecutive runs of 256 flattened elements.
 // A multi-tensor launch numbers the work items of all tensors of one mapping consecutively; a warp finds
 // its tensor by binary search in the prefix-sum table.  The step kernels are persistent: CTAs of 8 warps,
 // every warp striding over the item list.
@@ -17,8 +17,11 @@
 // Rank-1 second moments need the new row/column maxima of the whole tensor before any element can be
 // requantized, hence two passes: `pre` recomputes v from (g, old codes) and accumulates the maxima with
 // integer red.max on the bit patterns; `main` does the full update and recomputes the identical v to
-// quantize it against the finished maxima.  A small kernel in between stores the reciprocals of the new
-// maxima so that the main pass divides by multiplication plus exact residual correction.
+// quantize it against the finished maxima, whose reciprocals it takes once per item so that it divides by
+// multiplication plus exact residual correction.  A small kernel ahead of both clears the new maxima and
+// copies the old ones; the main pass reads the copy and stores the new maxima into the state beside its own
+// work, so that a step of matrices is three launches (five with separate passes for the reciprocals and for the
+// state: 4 + 25 + 20 us of small kernels on 645 M elements, now 5).
 //
 // Arithmetic.  The path is instruction-issue bound on B200 if written with the general IEEE division and
 // square-root expansions (about 135 instructions per element), so the hot loops use the packed-fp32
@@ -45,8 +48,8 @@ struct DevTensor {
     float* vcol;
     float* vrow_new;  // [rows]: new row maxima
     float* vcol_new;  // [cols]: new column maxima
-    float* vrow_rcp;  // [rows]: reciprocals of the new row maxima (NaN-tagged, see rank1_roll_kernel)
-    float* vcol_rcp;  // [cols]: the same for the columns
+    float* vrow_old;  // [rows]: copy of the old row maxima the second pass reads (it overwrites `vs` while it runs)
+    float* vcol_old;  // [cols]: the same for the columns
     int64_t numel;    // elements this record covers
     int64_t flat_off; // RANK1, flat mapping: elements of the matrix that precede this record's first one
     int32_t rows, cols;
@@ -54,7 +57,9 @@ struct DevTensor {
     int32_t flags;    // kFlagVec | kFlagPanel
     int32_t panels;   // panels per row band (cols / 256) for the panel mapping
     int32_t main_rows;  // panel mapping: rows of one item of the second pass (kMainRowsPerItem, or fewer on small launches)
-    int64_t pad1[3];
+    int32_t pre_rows;   // panel mapping: rows of one item of the first pass (kPreRowsPerItem, or fewer on small launches)
+    int32_t flat_runs;  // flat mapping: runs of 256 elements of one item (kRowsPerItem, or fewer on small launches)
+    int64_t pad1[2];
 };
 static_assert(sizeof(DevTensor) == 160, "DevTensor must stay 160 bytes");
 
@@ -243,6 +248,21 @@ __device__ __forceinline__ uint32_t byte_of(uint32_t w, int j) {
 __device__ __forceinline__ f2 widen_bf16x2(uint32_t w) {
     return mk2(__uint_as_float(prmt(w, 0u, 0x1044u)), __uint_as_float(prmt(w, 0u, 0x3244u)));
 }
+// The two 16-bit values of a word as floats, and back (nearest even).
+template <typename T>
+__device__ __forceinline__ f2 widen16(uint32_t w) {
+    if (std::is_same<T, __half>::value) return __half22float2(*reinterpret_cast<const __half2*>(&w));
+    return widen_bf16x2(w);
+}
+template <typename T>
+__device__ __forceinline__ uint32_t pack16(f2 x) {
+    if (std::is_same<T, __half>::value) {
+        const __half2 h = __floats2half2_rn(x.x, x.y);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    }
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x.x, x.y);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
 // ceil(y) as a signed integer (saturating; NaN gives 0).
 __device__ __forceinline__ int ceil_s32(float y) {
     int c;
@@ -412,7 +432,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // Panel mapping, rank-1 tensors
 // =================================================================================================
 
-// First pass over one item of a rank-1 panel.  This pass does little arithmetic per byte, so it needs many bytes in
+// First pass over one item of a rank-1 panel: the work of a whole CTA, each warp taking `pre_rows` consecutive rows of the
+// panel's 256 columns.  This pass does little arithmetic per byte, so it needs many bytes in
 // flight to cover HBM latency: each lane stages its own 16-byte piece of g and its code word of the next
 // kPreStages - 1 rows into a per-warp ring with cp.async (a lane reads only what it copied, so no barrier), and the
 // old row maxima of the item are fetched up front, two per lane, and handed out by shuffle.
@@ -421,13 +442,15 @@ constexpr int pre_dyn_smem(bool any_f32) { return kWarpsPerCta * kPreStages * 32
 
 template <typename T, bool SCALE>
 __device__ __forceinline__ void pre_panel(const DevTensor& t, int64_t li, const HyperDev& hd, const SmemPre& s,
-                                          char* stage, uint32_t* status) {
-    static_assert(kPreRowsPerItem == 64, "two old row maxima per lane");
+                                          char* stage, int ring_bytes, uint32_t* status) {
+    static_assert(kPanelCols == kThreads, "one column per thread in the combination of the warps' column maxima");
+    static_assert(kPreRowsPerItem <= 64, "two old row maxima per lane");
     const int lane = threadIdx.x & 31;
     const int band = static_cast<int>(li / t.panels);
     const int panel = static_cast<int>(li - static_cast<int64_t>(band) * t.panels);
-    const int r0 = band * kPreRowsPerItem;
-    const int r1 = min(r0 + kPreRowsPerItem, t.rows);
+    // the item's rows go to the CTA's warps in consecutive pieces; the last pieces of a tensor may be empty
+    const int r0 = min((band * kWarpsPerCta + static_cast<int>(threadIdx.x >> 5)) * t.pre_rows, t.rows);
+    const int r1 = min(r0 + t.pre_rows, t.rows);
     const int j0 = panel * kPanelCols + lane * 8;
     const uint8_t* vc = reinterpret_cast<const uint8_t*>(t.v);
     constexpr int NV = sizeof(T) / 2;
@@ -448,7 +471,7 @@ __device__ __forceinline__ void pre_panel(const DevTensor& t, int64_t li, const 
         e_issue += cols;
         ++r_issue;
     }
-    const float rows_lo = __ldg(t.vs + min(r0 + lane, r1 - 1)), rows_hi = __ldg(t.vs + min(r0 + 32 + lane, r1 - 1));
+    const float rows_lo = __ldg(t.vs + min(r0 + lane, t.rows - 1)), rows_hi = __ldg(t.vs + min(r0 + 32 + lane, t.rows - 1));
     float col_old[8];
     load8f(t.vcol, j0, col_old);
     const Hyper2 h2 = widen(hd);
@@ -513,28 +536,39 @@ __device__ __forceinline__ void pre_panel(const DevTensor& t, int64_t li, const 
     if (r0 + lane < r1) atomic_max_nonneg(t.vrow_new + r0 + lane, keep_lo);
     if (r0 + 32 + lane < r1) atomic_max_nonneg(t.vrow_new + r0 + 32 + lane, keep_hi);
     if (__any_sync(kFull, max(keep_lo, keep_hi) >= 0x7f800000u) && lane == 0) atomicOr(status, QF_STATUS_NONFINITE);
+    // Column maxima of the CTA's rows: every warp leaves its own in its (now idle) ring, then each thread takes one column
+    // over the eight warps: one atomic per column and item.
+    uint4* mine = reinterpret_cast<uint4*>(stage) + lane * 2;
+    mine[0] = make_uint4(cmax[0], cmax[1], cmax[2], cmax[3]);
+    mine[1] = make_uint4(cmax[4], cmax[5], cmax[6], cmax[7]);
+    __syncthreads();
+    const char* rings = stage - static_cast<int>(threadIdx.x >> 5) * ring_bytes;
+    uint32_t c = 0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) atomic_max_nonneg(t.vcol_new + j0 + k, cmax[k]);
+    for (int w = 0; w < kWarpsPerCta; ++w) c = max(c, *reinterpret_cast<const uint32_t*>(rings + w * ring_bytes + threadIdx.x * 4));
+    atomic_max_nonneg(t.vcol_new + panel * kPanelCols + threadIdx.x, c);
+    __syncthreads();   // the next item fills the rings again
 }
 
 // One row of a panel, exact arithmetic (also the reference for what the fast row must produce).  Kept out
-// of line and self-contained (it reloads its column maxima) so that it costs the hot loop no registers.
+// of line and self-contained (it reloads its column maxima) so that it costs the hot loop no registers.  Returns the
+// lane's new block scale; the caller stores it.
 template <typename T>
-__device__ __noinline__ void main_panel_row_exact(const DevTensor* tp, int64_t e, int r, int j0, const HyperDev& hd,
+__device__ __noinline__ float main_panel_row_exact(const DevTensor* tp, int64_t e, int r, int j0, const HyperDev& hd,
                                                   const Smem& s, uint32_t* status, const PushPack* push) {
     const DevTensor t = *tp;
     const int lane = threadIdx.x & 31;
     uint8_t* mc = reinterpret_cast<uint8_t*>(t.m);
     uint8_t* vc = reinterpret_cast<uint8_t*>(t.v);
     float p[8], g[8], m[8], v[8], col_old[8], col_new[8];
-    load8f(t.vcol, j0, col_old);
+    load8f(t.vcol_old, j0, col_old);
     load8f(t.vcol_new, j0, col_new);
     Elem<T>::load8(t.p, e, p);
     Elem<T>::load8(t.g, e, g);
     const uint32_t wm = *reinterpret_cast<const uint32_t*>(mc + (e >> 1));
     const uint32_t wv = *reinterpret_cast<const uint32_t*>(vc + (e >> 1));
     const float ms_old = __ldg(t.ms + (e >> 7));
-    const float row_old = __ldg(t.vs + r);
+    const float row_old = __ldg(t.vrow_old + r);
     const float row_new = t.vrow_new[r];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -546,14 +580,12 @@ __device__ __noinline__ void main_panel_row_exact(const DevTensor* tp, int64_t e
     if (push) push_store8<T>(t.p, e, p, push);
     const float ms_new = absmax8_bits_to_block(m);
     *reinterpret_cast<uint32_t*>(mc + (e >> 1)) = quantize8(m, ms_new, s.t.mm, 8);
-    if ((lane & 15) == 0) {
-        t.ms[e >> 7] = ms_new;
-        if (nonfinite(ms_new)) atomicOr(status, QF_STATUS_NONFINITE);
-    }
+    if ((lane & 15) == 0 && nonfinite(ms_new)) atomicOr(status, QF_STATUS_NONFINITE);
     uint32_t w = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) w |= search16(scaled(v[k], fminf(row_new, col_new[k])), s.t.mv) << (4 * k);
     *reinterpret_cast<uint32_t*>(vc + (e >> 1)) = w;
+    return ms_new;
 }
 
 // ---- asynchronous staging of the rows of a panel ---------------------------------------------------------
@@ -572,7 +604,10 @@ constexpr int kColBytes = 3 * 4 * 32 * 8;              // per warp: old / new / 
 // Dynamic shared memory of the panel kernel: per warp the two slots plus the column block.  The host sizes the
 // slots for fp32 rows only when the launch holds an fp32 panel tensor: less shared memory leaves more L1 to the
 // CTA, which the measurements reward.
-constexpr int main_dyn_smem(bool any_f32) { return kWarpsPerCta * (kStages * (any_f32 ? kRowBytesF32 : kRowBytesBf16) + kColBytes); }
+constexpr int kRowBufBytes = 2 * kMainRowsPerItem * 16;  // per warp: the scalars of every row of its item, once per 128-block
+constexpr int main_dyn_smem(bool any_f32) {
+    return kWarpsPerCta * (kStages * (any_f32 ? kRowBytesF32 : kRowBytesBf16) + kColBytes + kRowBufBytes);
+}
 
 // The AdamW update of two elements inside the panel loop (second moment at least 2^-94, see adamw_pair).  P1: the
 // two divisions of the parameter update with one residual correction (div2_prepared1 says what that means); taken for
@@ -602,8 +637,7 @@ __device__ __forceinline__ void adamw_pair_panel(f2& p, f2 g, f2& m, f2& v, cons
 // Second pass over one item of a rank-1 panel: 64 rows of 256 columns.
 //
 // The hot loop holds no call and stores nothing of a row before it knows that the whole row could take the packed
-// arithmetic: the row and column scalars inside the range of the division sequences (the pass that stored the
-// reciprocals wrote NaN where an old or a new maximum is not), old maxima above zero (a zero one, as on the first
+// arithmetic: the row and column scalars inside the range of the division sequences, old maxima above zero (a zero one, as on the first
 // step, lets the second moment fall below the range of the unchecked square root), the old block scale finite and
 // the new one zero or inside the range.  A row that fails leaves the loop untouched and is redone by
 // main_panel_row_exact from its unmodified inputs, after which the hot loop starts again behind it.  Rows go in
@@ -612,7 +646,8 @@ __device__ __forceinline__ void adamw_pair_panel(f2& p, f2 g, f2& m, f2& v, cons
 template <typename T, bool PUSH, bool BC1, bool RELAXED = false>
 __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, const HyperDev& hd, const Smem& s,
                                            char* stage, int ring_bytes, uint32_t* status, const PushPack* push) {
-    constexpr bool BF16 = std::is_same<T, __nv_bfloat16>::value;
+    constexpr bool BF16 = std::is_same<T, __nv_bfloat16>::value;   // its update takes one residual correction
+    constexpr bool H16 = sizeof(T) == 2;
     const DevTensor t = *tp;
     const int lane = threadIdx.x & 31;
     const int band = static_cast<int>(li / t.panels);
@@ -646,11 +681,13 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
     bool ok = hd.fast;
     {
         float col_old[8], col_new[8], rcol[8];
-        load8f(t.vcol, j0, col_old);
+        load8f(t.vcol_old, j0, col_old);
         load8f(t.vcol_new, j0, col_new);
-        load8f(t.vcol_rcp, j0, rcol);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) ok &= rcol[k] == rcol[k] && col_old[k] > 0.0f;
+        for (int k = 0; k < 8; ++k) {
+            rcol[k] = col_new[k] == 0.0f ? 0.0f : __frcp_rn(col_new[k]);
+            ok &= scale_safe(col_new[k]) && scale_safe(col_old[k]) && col_old[k] > 0.0f;
+        }
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             colbuf[(0 * 2 + j) * 32] = make_float4(col_old[4 * j], col_old[4 * j + 1], col_old[4 * j + 2], col_old[4 * j + 3]);
@@ -661,79 +698,31 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
     const bool col_fast = __all_sync(kFull, ok);
     const Hyper2 h2 = widen(hd);
 
-    struct RowScalars {
-        float ms_old, row_old, row_new, rrow;
-    };
-    auto fetch_scalars = [&](int r, uint32_t e) {
-        RowScalars o;
-        o.ms_old = ldg_early(t.ms + (e >> 7));
-        o.row_old = ldg_early(t.vs + r);
-        o.row_new = ldg_early(t.vrow_new + r);
-        o.rrow = ldg_early(t.vrow_rcp + r);
-        return o;
-    };
+    // The scalars of the item's rows: (old maximum, -new maximum, 1 / new maximum, old block scale), one entry per row
+    // and 128-block, fetched a row per lane and read back by the whole warp with one broadcast load per row (four
+    // global loads with their addresses per row before).  The reciprocal is NaN where the row cannot take the packed
+    // arithmetic: a maximum outside the range of the division sequences or an old maximum of zero.  The row's new
+    // block scale replaces the old one and goes out with the others at the end of the item.
+    float4* const rowbuf = reinterpret_cast<float4*>(stage + ring_bytes + kColBytes);
+    const uint32_t block0 = (static_cast<uint32_t>(r0) * cols + panel * kPanelCols) >> 7, row_blocks = cols >> 7;
+    for (int k = lane; k < r1 - r0; k += 32) {
+        const float old = __ldg(t.vrow_old + r0 + k), nw = __ldg(t.vrow_new + r0 + k);
+        const float* ms = t.ms + block0 + static_cast<uint32_t>(k) * row_blocks;
+        const float rr = nw == 0.0f ? 0.0f : __frcp_rn(nw);
+        const bool fit = scale_safe(nw) && scale_safe(old) && old > 0.0f;
+        float4 e4 = make_float4(old, -nw, fit ? rr : __uint_as_float(0x7fc00000u), ms[0]);
+        rowbuf[k] = e4;
+        e4.w = ms[1];
+        rowbuf[kMainRowsPerItem + k] = e4;
+    }
+    __syncwarp();
+    float4* const my_rows = rowbuf + (lane >> 4) * kMainRowsPerItem;   // the entries of this lane's 128-block
 
-    // One row out of the staging slot at `slot_off`.  False: the row cannot take the packed arithmetic; nothing of
-    // it has been stored.
-    auto row = [&](const RowScalars& sc, uint32_t e, int slot_off) -> bool {
-        // the staged row as it was copied: four words of two bf16 values, or eight floats, per array
-        uint32_t pw[NV * 4], gw[NV * 4];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const uint4 a = *reinterpret_cast<const uint4*>(lane_vec + slot_off + v * 512);
-            const uint4 b = *reinterpret_cast<const uint4*>(lane_vec + slot_off + kArr + v * 512);
-            pw[4 * v] = a.x; pw[4 * v + 1] = a.y; pw[4 * v + 2] = a.z; pw[4 * v + 3] = a.w;
-            gw[4 * v] = b.x; gw[4 * v + 1] = b.y; gw[4 * v + 2] = b.z; gw[4 * v + 3] = b.w;
-        }
-        f2 pp[4];
-        const uint32_t wm = *reinterpret_cast<const uint32_t*>(lane_codes + slot_off);
-        const uint32_t wv = *reinterpret_cast<const uint32_t*>(lane_codes + slot_off + 128);
-        const f2 ms_old = bc2(sc.ms_old);
-        const float row_old = sc.row_old, nrow = -sc.row_new, rrow = sc.rrow;
-        f2 m[4];
-        int cv[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            pp[j] = BF16 ? widen_bf16x2(pw[j]) : mk2(__uint_as_float(pw[(2 * j) % (NV * 4)]), __uint_as_float(pw[(2 * j + 1) % (NV * 4)]));
-            const f2 gg = BF16 ? widen_bf16x2(gw[j]) : mk2(__uint_as_float(gw[(2 * j) % (NV * 4)]), __uint_as_float(gw[(2 * j + 1) % (NV * 4)]));
-            m[j] = mul2(pair_entry(s.qm2, wm, j), ms_old);
-            const float4 a = colbuf[(0 * 2 + (j >> 1)) * 32], b = colbuf[(1 * 2 + (j >> 1)) * 32], c = colbuf[(2 * 2 + (j >> 1)) * 32];
-            const f2 co = (j & 1) ? mk2(a.z, a.w) : mk2(a.x, a.y);
-            const f2 ncn = (j & 1) ? mk2(b.z, b.w) : mk2(b.x, b.y);
-            const f2 rcn = (j & 1) ? mk2(c.z, c.w) : mk2(c.x, c.y);
-            f2 v = mul2(pair_entry(s.qv2, wv, j), mk2(fminf(row_old, co.x), fminf(row_old, co.y)));
-            adamw_pair_panel<BF16, BC1, RELAXED>(pp[j], gg, m[j], v, h2);
-            // requantize v: scale = min(row', col') -> -scale = max(-row', -col'), 1/scale = max(1/row', 1/col')
-            const f2 nsv = mk2(fmaxf(nrow, ncn.x), fmaxf(nrow, ncn.y));
-            const f2 rv = mk2(fmaxf(rrow, rcn.x), fmaxf(rrow, rcn.y));
-            const f2 y = fma2(div2_prepared1(v, rv, nsv), bc2(16.0f), bc2(-1.5f));
-            cv[2 * j] = ceil_s32(y.x);       // x <= 1 here (the scale is a maximum over values that include v): at most 15
-            cv[2 * j + 1] = ceil_s32(y.y);
-        }
-        const float ms_new = absmax_pairs_to_block(m);
-        const bool row_ok = sc.rrow == sc.rrow && sc.row_old > 0.0f && sc.ms_old < __builtin_huge_valf() && scale_safe(ms_new);
-        if (!__all_sync(kFull, row_ok)) return false;     // the vote also tells the compiler that the branch is uniform
-        uint32_t wmq;
-        {
-            const Recip rc = make_recip(ms_new);  // 0 for an all-zero block: every quotient is 0
-            const f2 r2 = bc2(rc.r), ns2 = bc2(rc.nd);
-            int c[8];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const f2 q = div2_prepared1(m[j], r2, ns2);
-                c[2 * j] = search_m_lut(q.x, s.mlut, s.t.mm);
-                c[2 * j + 1] = search_m_lut(q.y, s.mlut, s.t.mm);
-            }
-            wmq = pack_u4(c[1], c[0], pack_u4(c[3], c[2], pack_u4(c[5], c[4], pack_u4(c[7], c[6], 0u))));
-        }
-        const uint32_t wq = pack_u4(cv[1], cv[0], pack_u4(cv[3], cv[2], pack_u4(cv[5], cv[4], pack_u4(cv[7], cv[6], 0u))));
-        if (BF16) {
+    auto store_p = [&](uint32_t e, const f2 (&pp)[4]) {
+        if (H16) {
             uint32_t w[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(pp[j].x, pp[j].y);  // nearest even
-                w[j] = *reinterpret_cast<const uint32_t*>(&h);
-            }
+            for (int j = 0; j < 4; ++j) w[j] = pack16<T>(pp[j]);
             const uint4 out = make_uint4(w[0], w[1], w[2], w[3]);
             *reinterpret_cast<uint4*>(t.p + static_cast<size_t>(e) * 2) = out;
             if (PUSH) {
@@ -754,9 +743,87 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
                 }
             }
         }
+    };
+
+    // One row out of the staging slot at `slot_off`.  False: the row cannot take the packed arithmetic; nothing of
+    // it has been stored.
+    auto row = [&](int k_row, uint32_t e, int slot_off) -> bool {
+        const float4 sc = my_rows[k_row];
+        // the staged row as it was copied: four words of two bf16 values, or eight floats, per array
+        uint32_t pw[NV * 4], gw[NV * 4];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const uint4 a = *reinterpret_cast<const uint4*>(lane_vec + slot_off + v * 512);
+            const uint4 b = *reinterpret_cast<const uint4*>(lane_vec + slot_off + kArr + v * 512);
+            pw[4 * v] = a.x; pw[4 * v + 1] = a.y; pw[4 * v + 2] = a.z; pw[4 * v + 3] = a.w;
+            gw[4 * v] = b.x; gw[4 * v + 1] = b.y; gw[4 * v + 2] = b.z; gw[4 * v + 3] = b.w;
+        }
+        f2 pp[4];
+        const uint32_t wm = *reinterpret_cast<const uint32_t*>(lane_codes + slot_off);
+        const uint32_t wv = *reinterpret_cast<const uint32_t*>(lane_codes + slot_off + 128);
+        const f2 ms_old = bc2(sc.w);
+        const float row_old = sc.x, nrow = sc.y, rrow = sc.z;
+        f2 m[4];
+        if (__any_sync(kFull, row_old == 0.0f)) {
+            // A row without second moment (a token that has not occurred, the padding of a vocabulary): where its first
+            // moment and its gradient are zero as well, the moments stay zero -- codes of x = 0, scale 0 -- and the
+            // parameter only decays (the quotient of the update is a zero of the first moment's sign).
+            uint32_t any = __float_as_uint(sc.w);
+#pragma unroll
+            for (int j = 0; j < NV * 4; ++j) any |= gw[j] & (H16 ? 0x7fff7fffu : 0x7fffffffu);
+            if (__any_sync(kFull, any != 0)) return false;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const f2 p0 = H16 ? widen16<T>(pw[j]) : mk2(__uint_as_float(pw[(2 * j) % (NV * 4)]), __uint_as_float(pw[(2 * j + 1) % (NV * 4)]));
+                const f2 gg = H16 ? widen16<T>(gw[j]) : mk2(__uint_as_float(gw[(2 * j) % (NV * 4)]), __uint_as_float(gw[(2 * j + 1) % (NV * 4)]));
+                const f2 mo = mul2(pair_entry(s.qm2, wm, j), ms_old);
+                pp[j] = fma2(h2.nstep, fma2(h2.w1, add2(gg, neg2(mo)), mo), fma2(p0, h2.decay, bc2(-0.0f)));  // -0 keeps the sign of a zero parameter
+            }
+            store_p(e, pp);
+            *reinterpret_cast<uint32_t*>(vc + (e >> 1)) = 0u;
+            *reinterpret_cast<uint32_t*>(mc + (e >> 1)) = 0x77777777u;
+            return true;     // the block scale stays zero
+        }
+        int cv[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            pp[j] = H16 ? widen16<T>(pw[j]) : mk2(__uint_as_float(pw[(2 * j) % (NV * 4)]), __uint_as_float(pw[(2 * j + 1) % (NV * 4)]));
+            const f2 gg = H16 ? widen16<T>(gw[j]) : mk2(__uint_as_float(gw[(2 * j) % (NV * 4)]), __uint_as_float(gw[(2 * j + 1) % (NV * 4)]));
+            m[j] = mul2(pair_entry(s.qm2, wm, j), ms_old);
+            const float4 a = colbuf[(0 * 2 + (j >> 1)) * 32], b = colbuf[(1 * 2 + (j >> 1)) * 32], c = colbuf[(2 * 2 + (j >> 1)) * 32];
+            const f2 co = (j & 1) ? mk2(a.z, a.w) : mk2(a.x, a.y);
+            const f2 ncn = (j & 1) ? mk2(b.z, b.w) : mk2(b.x, b.y);
+            const f2 rcn = (j & 1) ? mk2(c.z, c.w) : mk2(c.x, c.y);
+            f2 v = mul2(pair_entry(s.qv2, wv, j), mk2(fminf(row_old, co.x), fminf(row_old, co.y)));
+            adamw_pair_panel<BF16, BC1, RELAXED>(pp[j], gg, m[j], v, h2);
+            // requantize v: scale = min(row', col') -> -scale = max(-row', -col'), 1/scale = max(1/row', 1/col')
+            const f2 nsv = mk2(fmaxf(nrow, ncn.x), fmaxf(nrow, ncn.y));
+            const f2 rv = mk2(fmaxf(rrow, rcn.x), fmaxf(rrow, rcn.y));
+            const f2 y = fma2(div2_prepared1(v, rv, nsv), bc2(16.0f), bc2(-1.5f));
+            cv[2 * j] = ceil_s32(y.x);       // x <= 1 here (the scale is a maximum over values that include v): at most 15
+            cv[2 * j + 1] = ceil_s32(y.y);
+        }
+        const float ms_new = absmax_pairs_to_block(m);
+        const bool row_ok = rrow == rrow && sc.w < __builtin_huge_valf() && scale_safe(ms_new);
+        if (!__all_sync(kFull, row_ok)) return false;     // the vote also tells the compiler that the branch is uniform
+        uint32_t wmq;
+        {
+            const Recip rc = make_recip(ms_new);  // 0 for an all-zero block: every quotient is 0
+            const f2 r2 = bc2(rc.r), ns2 = bc2(rc.nd);
+            int c[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const f2 q = div2_prepared1(m[j], r2, ns2);
+                c[2 * j] = search_m_lut(q.x, s.mlut, s.t.mm);
+                c[2 * j + 1] = search_m_lut(q.y, s.mlut, s.t.mm);
+            }
+            wmq = pack_u4(c[1], c[0], pack_u4(c[3], c[2], pack_u4(c[5], c[4], pack_u4(c[7], c[6], 0u))));
+        }
+        const uint32_t wq = pack_u4(cv[1], cv[0], pack_u4(cv[3], cv[2], pack_u4(cv[5], cv[4], pack_u4(cv[7], cv[6], 0u))));
+        store_p(e, pp);
         *reinterpret_cast<uint32_t*>(vc + (e >> 1)) = wq;
         *reinterpret_cast<uint32_t*>(mc + (e >> 1)) = wmq;
-        if ((lane & 15) == 0) t.ms[e >> 7] = ms_new;
+        if ((lane & 15) == 0) my_rows[k_row].w = ms_new;
         return true;
     };
 
@@ -766,23 +833,20 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
             uint32_t e = static_cast<uint32_t>(r) * cols + j0;
             issue(e, 0);
             cp_async_commit();
-            RowScalars sa = fetch_scalars(r, e);
             // rows r (slot 0) and r + 1 (slot 1) per turn; row r is on its way when the turn starts
             for (; r + 1 < r1; r += 2, e += 2 * cols) {
                 issue(e + cols, kRowBytes);
                 cp_async_commit();
-                const RowScalars sb = fetch_scalars(r + 1, e + cols);
                 cp_async_wait<1>();  // everything but the newest group has landed
-                if (!row(sa, e, 0)) break;
-                // The row behind the pair goes into slot 0.  Past the end the last row is staged and its scalars are
-                // fetched again (nobody reads them): cheaper than a branch around the copies.
+                if (!row(r - r0, e, 0)) break;
+                // The row behind the pair goes into slot 0.  Past the end the last row is staged again (nobody reads it):
+                // cheaper than a branch around the copies.
                 const bool more = r + 2 < r1;
                 const uint32_t e2 = more ? e + 2 * cols : e + cols;
                 issue(e2, 0);
                 cp_async_commit();
-                sa = fetch_scalars(more ? r + 2 : r + 1, e2);
                 cp_async_wait<1>();
-                if (!row(sb, e + cols, kRowBytes)) {
+                if (!row(r + 1 - r0, e + cols, kRowBytes)) {
                     ++r;
                     break;
                 }
@@ -790,10 +854,18 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
             cp_async_wait<0>();
         }
         if (r < r1) {  // cold: this row exactly, from its unmodified inputs
-            main_panel_row_exact<T>(tp, static_cast<uint32_t>(r) * cols + j0, r, j0, hd, s, status, PUSH ? push : nullptr);
+            const float ms_new = main_panel_row_exact<T>(tp, static_cast<uint32_t>(r) * cols + j0, r, j0, hd, s, status, PUSH ? push : nullptr);
+            if ((lane & 15) == 0) my_rows[r - r0].w = ms_new;
             ++r;
         }
     }
+    __syncwarp();
+    for (int k = lane; k < r1 - r0; k += 32) {
+        float* ms = t.ms + block0 + static_cast<uint32_t>(k) * row_blocks;
+        ms[0] = rowbuf[k].w;
+        ms[1] = rowbuf[kMainRowsPerItem + k].w;
+    }
+    __syncwarp();   // the next item of this warp fills the buffer again
 }
 
 // =================================================================================================
@@ -857,9 +929,9 @@ __device__ __forceinline__ void pre_flat_rank1(const DevTensor& t, int64_t li, c
                                                uint32_t* status) {
     const int lane = threadIdx.x & 31;
     const bool vec = t.flags & kFlagVec;
-    const int64_t start = li * (kPanelCols * kRowsPerItem);
+    const int64_t start = li * (static_cast<int64_t>(kPanelCols) * t.flat_runs);
     const uint8_t* vc = reinterpret_cast<const uint8_t*>(t.v);
-    for (int it = 0; it < kRowsPerItem; ++it) {
+    for (int it = 0; it < t.flat_runs; ++it) {
         const int64_t wbase = start + static_cast<int64_t>(it) * kPanelCols;
         if (wbase >= t.numel) break;
         const int64_t e = wbase + lane * 8;
@@ -925,7 +997,7 @@ __device__ __noinline__ void main_flat_run_exact(const DevTensor* tp, int64_t wb
 #pragma unroll
         for (int k = 0; k < 8; ++k) sc_old[k] = sc_new[k] = 0.0f;
         if (nv) {
-            rank1_scales(t.vs, t.vcol, e + t.flat_off, nv, t.cols, sc_old, ri, ci);
+            rank1_scales(t.vrow_old, t.vcol_old, e + t.flat_off, nv, t.cols, sc_old, ri, ci);
             rank1_scales(t.vrow_new, t.vcol_new, e + t.flat_off, nv, t.cols, sc_new, ri, ci);
         }
     }
@@ -1035,9 +1107,9 @@ __device__ __forceinline__ void main_flat(const DevTensor* tp, int64_t li, const
                                           uint32_t* status, const PushPack* push) {
     const DevTensor t = *tp;
     const bool vec = t.flags & kFlagVec;
-    const int64_t start = li * (kPanelCols * kRowsPerItem);
+    const int64_t start = li * (static_cast<int64_t>(kPanelCols) * t.flat_runs);
     const Hyper2 h2 = widen(hd);
-    for (int it = 0; it < kRowsPerItem; ++it) {
+    for (int it = 0; it < t.flat_runs; ++it) {
         const int64_t wbase = start + static_cast<int64_t>(it) * kPanelCols;
         if (wbase >= t.numel) break;  // warp-uniform
         if (KIND != QF_KIND_RANK1 && hd.gs != 1.0f) {  // no first pass for these kinds: the gradient is scaled here
@@ -1054,6 +1126,38 @@ __device__ __forceinline__ void main_flat(const DevTensor* tp, int64_t li, const
         else
             main_flat_run_exact<T, KIND>(tp, wbase, hd, s, status, push);
     }
+}
+
+// Small passes over the row / column maxima of every rank-1 tensor, as bits of `mode`:
+//   kRollClear     new maxima := 0                        (before the first pass)
+//   kRollKeep      copy of the stored maxima for the second pass
+// An item is kRollEntries consecutive entries (rows, then columns) of one tensor; `base` is the prefix-sum table of the
+// items.  One CTA per item: with four CTAs per tensor instead, an embedding of 32 000 rows walked 37 dependent
+// turns and the pass took 17 .. 25 us.
+constexpr int kRollEntries = 4 * kThreads;
+enum { kRollClear = 1, kRollKeep = 2, kRollCommit = 4 };
+__device__ __forceinline__ void roll_item(const DevTensor* __restrict__ tensors, const int64_t* __restrict__ base, int n, int64_t item,
+                                          int mode) {
+    const int ti = find_tensor(base, n, item);
+    const DevTensor& t = tensors[ti];
+    const int rows = t.rows, total = rows + t.cols;
+    const int64_t first = (item - base[ti]) * kRollEntries + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < kRollEntries / kThreads; ++k) {
+        const int64_t i = first + k * kThreads;
+        if (i >= total) continue;
+        const bool is_row = i < rows;
+        const int64_t j = is_row ? i : i - rows;
+        float* now = is_row ? t.vs : t.vcol;
+        float* fresh = is_row ? t.vrow_new : t.vcol_new;
+        if (mode & kRollKeep) (is_row ? t.vrow_old : t.vcol_old)[j] = now[j];
+        if (mode & kRollClear) fresh[j] = 0.0f;
+        if (mode & kRollCommit) now[j] = fresh[j];
+    }
+}
+__global__ void __launch_bounds__(kThreads)
+rank1_roll_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict__ base, int n, int mode) {
+    roll_item(tensors, base, n, blockIdx.x, mode);
 }
 
 // =================================================================================================
@@ -1077,17 +1181,19 @@ step_pre_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict
     load_smem(s);
     extern __shared__ __align__(16) char staging[];  // panel kernel: one ring of rows per warp
     char* stage = staging + (threadIdx.x >> 5) * ring_bytes;
-    const int64_t total = base[n], stride = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
-    for (int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5); item < total; item += stride) {
+    const int64_t total = base[n], per_cta = PANEL ? 1 : kWarpsPerCta, stride = gridDim.x * per_cta;
+    for (int64_t item = blockIdx.x * per_cta + (PANEL ? 0 : threadIdx.x >> 5); item < total; item += stride) {
         const int ti = find_tensor(base, n, item);
         const DevTensor t = tensors[ti];
         const int64_t li = item - base[ti];
         const HyperDev& h = SCHED ? sched_h[t.hyper] : hp.h[t.hyper];
         if (PANEL) {
             if (t.dtype == QF_BF16)
-                pre_panel<__nv_bfloat16, SCALE>(t, li, h, s, stage, status);
+                pre_panel<__nv_bfloat16, SCALE>(t, li, h, s, stage, ring_bytes, status);
+            else if (t.dtype == QF_F16)
+                pre_panel<__half, SCALE>(t, li, h, s, stage, ring_bytes, status);
             else
-                pre_panel<float, SCALE>(t, li, h, s, stage, status);
+                pre_panel<float, SCALE>(t, li, h, s, stage, ring_bytes, status);
         } else {
             if (t.dtype == QF_BF16)
                 pre_flat_rank1<__nv_bfloat16>(t, li, h, s, status);
@@ -1116,20 +1222,22 @@ constexpr int kMainMinCtas = 2;  // CTAs per SM the second pass is compiled for 
 // BC1 (panel mapping only): every hyper-parameter set of the launch has bc2s == 1.
 // SCHED: the hyper-parameter sets come from the device-resident table `sc` instead of `hp`.
 // RELAXED (panel mapping, bf16 tensors): the uncorrected parameter update of adamw_pair_panel.
-// DT (panel mapping): 0 = tensors of both dtypes, 1 = the launch holds bf16 panel tensors only, 2 = fp32 only; a kernel
-// that carries one dtype's loop is scheduled a little better than one that carries both.
+// DT (panel mapping): 0 = tensors of several dtypes, 1 = the launch holds bf16 panel tensors only, 2 = fp32 only, 3 = fp16
+// only; a kernel that carries one dtype's loop is scheduled a little better than one that carries all.
+// Every CTA ends with its share of the `n_roll` items that store the new row / column maxima (kRollCommit): the second
+// pass reads the old ones from the copies, so nothing has to wait for them.
 template <bool PANEL, bool PUSH, bool BC1 = false, bool SCHED = false, bool RELAXED = false, int DT = 0>
 __global__ void __launch_bounds__(kThreads, kMainMinCtas)
 step_main_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict__ base, int n,
                  const __grid_constant__ HyperPack hp, int ring_bytes, uint32_t* status,
-                 const __grid_constant__ PushPack pp, const __grid_constant__ Sched sc) {
+                 const __grid_constant__ PushPack pp, const __grid_constant__ Sched sc, const int64_t* __restrict__ roll_base, int n_roll) {
     const PushPack* push = PUSH ? &pp : nullptr;
     __shared__ Smem s;
     __shared__ HyperDev sched_h[SCHED ? QF_MAX_HYPERS : 1];
     if (SCHED) load_sched(sched_h, sc);
     load_smem(s);
     extern __shared__ __align__(16) char staging[];  // panel kernel: per warp a ring of rows plus the column block
-    char* stage = staging + (threadIdx.x >> 5) * (ring_bytes + kColBytes);
+    char* stage = staging + (threadIdx.x >> 5) * (ring_bytes + kColBytes + kRowBufBytes);
     const int64_t total = base[n], stride = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
     for (int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5); item < total; item += stride) {
         const int ti = find_tensor(base, n, item);
@@ -1139,6 +1247,8 @@ step_main_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restric
         if (PANEL) {
             if (DT == 1 || (DT == 0 && tp->dtype == QF_BF16))
                 main_panel<__nv_bfloat16, PUSH, BC1, RELAXED>(tp, li, h, s, stage, ring_bytes, status, push);
+            else if (DT == 3 || (DT == 0 && tp->dtype == QF_F16))
+                main_panel<__half, PUSH, BC1>(tp, li, h, s, stage, ring_bytes, status, push);
             else
                 main_panel<float, PUSH, BC1>(tp, li, h, s, stage, ring_bytes, status, push);
         } else {
@@ -1150,6 +1260,7 @@ step_main_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restric
                 main_flat_dispatch<float>(tp, li, h, s, status, push);
         }
     }
+    for (int i = blockIdx.x; i < n_roll; i += gridDim.x) roll_item(tensors, roll_base, n, i, kRollCommit);
 }
 
 // One tensor passed by value (the single-tensor entry points that mirror the reference's per-tensor
@@ -1160,7 +1271,7 @@ single_tensor_kernel(const __grid_constant__ DevTensor t, const __grid_constant_
     __shared__ Smem s;
     load_smem(s);
     const int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
-    if (item * (kPanelCols * kRowsPerItem) >= t.numel) return;
+    if (item * (static_cast<int64_t>(kPanelCols) * t.flat_runs) >= t.numel) return;
     if (t.dtype == QF_BF16)
         main_flat_dispatch<__nv_bfloat16>(&t, item, h, s, &g_unread_status, nullptr);
     else if (t.dtype == QF_F16)
@@ -1221,37 +1332,6 @@ __global__ void sched_advance_kernel(int32_t* counters, int rows, int tail_repea
     if (r >= rows && !tail_repeats) atomicOr(status, QF_STATUS_SCHEDULE_END);
     counters[0] = r < rows ? r + 1 : rows;
     counters[1] += 1;
-}
-
-// Small passes over the row / column maxima of every rank-1 tensor.  One CTA per (tensor, slice).
-//   kRollClear     new maxima := 0                       (before the first pass)
-//   kRollRecip     reciprocals of the new maxima         (between the passes; 0 for a zero maximum, NaN
-//                  where the old or the new maximum is outside the range of the fast division)
-//   kRollCommit    stored maxima := new maxima           (after the second pass)
-constexpr int kRollSlices = 4;
-enum { kRollClear = 0, kRollRecip = 1, kRollCommit = 2 };
-__global__ void __launch_bounds__(kThreads)
-rank1_roll_kernel(const DevTensor* __restrict__ tensors, int n, int mode) {
-    const int ti = blockIdx.x / kRollSlices;
-    if (ti >= n) return;
-    const DevTensor& t = tensors[ti];
-    if (t.kind != QF_KIND_RANK1) return;
-    const int total = t.rows + t.cols;
-    for (int i = (blockIdx.x % kRollSlices) * kThreads + threadIdx.x; i < total; i += kRollSlices * kThreads) {
-        const bool is_row = i < t.rows;
-        const int k = is_row ? i : i - t.rows;
-        float* nw = is_row ? t.vrow_new : t.vcol_new;
-        float* rcp = is_row ? t.vrow_rcp : t.vcol_rcp;
-        if (mode == kRollClear) {
-            nw[k] = 0.0f;
-        } else if (mode == kRollRecip) {
-            const float x = nw[k], old = (is_row ? t.vs : t.vcol)[k];
-            const float r = x == 0.0f ? 0.0f : __frcp_rn(x);
-            rcp[k] = scale_safe(x) && scale_safe(old) ? r : __uint_as_float(0x7fc00000u);
-        } else {
-            (is_row ? t.vs : t.vcol)[k] = nw[k];
-        }
-    }
 }
 
 // =================================================================================================

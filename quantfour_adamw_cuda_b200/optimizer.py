@@ -80,8 +80,7 @@ class FourBitAdamW(torch.optim.Optimizer):
     unsigned linear map without zero; for 2-D parameters the scale of element (i, j) is
     min(row_max[i], col_max[j]) (rank-1 normalisation), otherwise one scale per 128 elements.
     Parameters with at most ``quant_threshold`` elements keep float32 moments.  Parameters and
-    gradients must be CUDA tensors of dtype float32 or bfloat16; float16 works as well, through the kernels' general
-    (slower) element mapping.
+    gradients must be CUDA tensors of dtype float32, bfloat16 or float16.
     """
 
     def __init__(
@@ -172,7 +171,7 @@ class FourBitAdamW(torch.optim.Optimizer):
         s = self._scratch.get(p)
         if s is None or s[0].device != p.device:
             R, Cc = p.numel() // p.shape[-1], p.shape[-1]
-            # new maxima followed by their reciprocals (the layout qf_step_multi expects)
+            # new maxima followed by a copy of the old ones (the layout qf_step_multi expects)
             s = (torch.zeros(2 * R, dtype=torch.float32, device=p.device),
                  torch.zeros(2 * Cc, dtype=torch.float32, device=p.device))
             self._scratch[p] = s

@@ -1,0 +1,55 @@
+"""Bit-exact parity of the step kernels' dispatch branches at the sizes where they can go wrong, against the C oracle."""
+import pytest
+import torch
+
+from helpers import AbiStepper, GpuState, make_grad
+from oracle import c_oracle as CO
+from oracle import torch_oracle as TO
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+HP = dict(lr=1e-3, betas=(0.9, 0.999), eps=1e-8, weight_decay=0.01)
+ARGS = (HP["lr"], *HP["betas"], HP["eps"], HP["weight_decay"])
+
+
+def run(specs, steps=4, dead_rows=0.0, seed=0):
+    """A few free-running steps of a list of tensors; everything must equal the oracle bit for bit.  `dead_rows`: the share
+    of a matrix's rows whose gradient is zero (of either sign) until the last step."""
+    gen = torch.Generator().manual_seed(seed)
+    params = [(torch.randn(s, generator=gen) * 0.02).to(dt) for s, dt in specs]
+    for p in params:
+        p.view(-1)[:2] = torch.tensor([0.0, -0.0], dtype=p.dtype)[:p.numel()]
+    ostates = [TO.TensorState.zeros(s) for s, _ in specs]
+    gparams = [p.to(DEV) for p in params]
+    gstates = [GpuState(st) for st in ostates]
+    stepper = AbiStepper(gparams, gstates, **HP)
+    gone = [torch.rand([s[0]] + [1] * (len(s) - 1), generator=gen) < dead_rows for s, _ in specs]
+    for step in range(steps):
+        grads = [make_grad(p.shape, p.dtype, gen=gen) for p in params]
+        if dead_rows and step + 1 < steps:
+            grads = [torch.where(d, g * 0, g) for d, g in zip(gone, grads)]
+        for p, g, st in zip(params, grads, ostates):
+            CO.step_tensor(p, g, st, *ARGS)
+        stepper.step([g.to(DEV) for g in grads], split=step % 2 == 1)
+        for i, (p, st, gp, gs) in enumerate(zip(params, ostates, gparams, gstates)):
+            what = f"step {step + 1} tensor {i} {tuple(p.shape)} {p.dtype}"
+            assert torch.equal(gp.cpu(), p), what
+            assert torch.equal(torch.signbit(gp.cpu()), torch.signbit(p)), what
+            assert not any(gs.diff(st).values()), f"{what}: {gs.diff(st)}"
+    assert stepper.status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows", [17, 127, 129, 513])
+def test_panels_of_odd_row_counts(dtype, rows):
+    run([((rows, 256), dtype), ((rows, 1024), dtype)])
+
+
+def test_panels_of_several_dtypes_in_one_launch():
+    run([((200, 256), torch.float16), ((131, 512), torch.bfloat16), ((64, 768), torch.float32), ((5000,), torch.float16)])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_rows_without_state_and_gradient(dtype):
+    run([((130, 512), dtype), ((257, 256), dtype)], dead_rows=0.5)
