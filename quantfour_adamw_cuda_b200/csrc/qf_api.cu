@@ -38,7 +38,7 @@ int fail(int code, const char* fmt, ...) {
 
 constexpr size_t kStatusBytes = 256;  // head of the workspace: status word, then padding
 
-constexpr int kTables = 5;  // prefix sums: main/panel, main/flat, pre/panel, pre/flat, row and column maxima
+constexpr int kTables = 6;  // prefix sums: main/panel, main/flat, pre/panel, pre/flat, row and column maxima, strips (both passes)
 size_t table_bytes(int n) { return static_cast<size_t>(n) * sizeof(qf::DevTensor) + kTables * (static_cast<size_t>(n) + 1) * 8; }
 size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -93,7 +93,7 @@ bool drop_cache_entry(WsCache& c, bool wait) {
     return true;
 }
 
-enum { kMainPanel = 0, kMainFlat = 1, kPrePanel = 2, kPreFlat = 3, kRoll = 4 };
+enum { kMainPanel = 0, kMainFlat = 1, kPrePanel = 2, kPreFlat = 3, kRoll = 4, kStrip = 5 };
 struct Plan {
     int n = 0;                    // tensors in the table (zero-size tensors dropped)
     int64_t items[kTables] = {};
@@ -121,6 +121,12 @@ int main_rows_for(int64_t items) {
 // two CTA items per slot: 512 rows per item left the device a ragged last wave (202 M elements: 139 -> 125 us)
 int pre_rows_for(int64_t items) { return item_length(items, qf::kPreRowsPerItem, qf::kMinPreRowsPerItem, 2 * qf::kPreMinCtas); }
 int flat_runs_for(int64_t items) { return item_length(items, qf::kRowsPerItem, qf::kMinRowsPerItem, qf::kMainMinCtas * qf::kWarpsPerCta); }
+
+// Strips: two CTAs' worth per SM of the shortest length, as for the other mappings.
+int strip_runs_for(int64_t items) { return item_length(items, qf::kStripRuns, 1, qf::kMainMinCtas); }
+// The strip mapping takes a rank-1 tensor that is not whole panels if its buffers are vector-aligned and a lane's eight
+// elements cross at most one row end.
+bool strip_fits(int64_t cols, bool vec) { return vec && cols >= 8; }
 
 int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* workspace, size_t workspace_bytes,
                int device, cudaStream_t stream, Plan* plan, bool upload = true) {
@@ -198,37 +204,45 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
                 if (d.dtype == QF_F32) plan->any_f32_panel = true;
                 if (d.dtype == QF_BF16) plan->any_bf16_panel = true;
                 if (d.dtype == QF_F16) plan->any_f16_panel = true;
+            } else if (strip_fits(d.cols, vec)) {
+                t.flags |= qf::kFlagStrip;
             }
             ++n_rank1;
         }
         if (vec) t.flags |= qf::kFlagVec;
-        const bool panel = t.flags & qf::kFlagPanel, rank1 = d.kind == QF_KIND_RANK1;
+        const bool panel = t.flags & qf::kFlagPanel, strip = t.flags & qf::kFlagStrip, rank1 = d.kind == QF_KIND_RANK1;
+        // items of the longest form; shorter ones are chosen below from these sums
         base[kMainPanel].push_back(base[kMainPanel].back() + (panel ? items : 0));
-        base[kMainFlat].push_back(base[kMainFlat].back() + (panel ? 0 : items));
-        base[kPrePanel].push_back(base[kPrePanel].back() + (rank1 && panel ? pre_items : 0));
-        base[kPreFlat].push_back(base[kPreFlat].back() + (rank1 && !panel ? pre_items : 0));
+        base[kMainFlat].push_back(base[kMainFlat].back() + (panel || strip ? 0 : items));
+        base[kPrePanel].push_back(base[kPrePanel].back() + (panel ? pre_items : 0));
+        base[kPreFlat].push_back(0);
         base[kRoll].push_back(base[kRoll].back() + (rank1 ? ceil_div(d.rows + d.cols, qf::kRollEntries) : 0));
+        base[kStrip].push_back(base[kStrip].back() + (strip ? ceil_div(d.numel, qf::strip_entries(qf::kStripRuns)) : 0));
         tab.push_back(t);
     }
     const int n = static_cast<int>(tab.size());
     // a small launch: shorter items, so that the whole device takes part
     const int main_rows = main_rows_for(base[kMainPanel].back()), pre_rows = pre_rows_for(base[kPrePanel].back());
-    const int flat_runs = flat_runs_for(base[kMainFlat].back());
+    const int flat_runs = flat_runs_for(base[kMainFlat].back()), strip_runs = strip_runs_for(base[kStrip].back());
     int64_t acc[kTables] = {};
     for (int i = 0; i < n; ++i) {
         qf::DevTensor& t = tab[i];
         t.main_rows = main_rows;
         t.pre_rows = pre_rows;
         t.flat_runs = flat_runs;
+        t.strip_runs = strip_runs;
         if (t.flags & qf::kFlagPanel) {
             acc[kMainPanel] += ceil_div(t.rows, main_rows) * t.panels;
             acc[kPrePanel] += ceil_div(t.rows, pre_rows * qf::kWarpsPerCta) * t.panels;
+        } else if (t.flags & qf::kFlagStrip) {
+            acc[kStrip] += ceil_div(t.numel, qf::strip_entries(strip_runs));
         } else {
             const int64_t items = ceil_div(t.numel, static_cast<int64_t>(qf::kPanelCols) * flat_runs);
             acc[kMainFlat] += items;
             if (t.kind == QF_KIND_RANK1) acc[kPreFlat] += items;
         }
-        for (int k = 0; k < kRoll; ++k) base[k][i + 1] = acc[k];
+        acc[kRoll] = base[kRoll][i + 1];
+        for (int k = 0; k < kTables; ++k) base[k][i + 1] = acc[k];
     }
     plan->n = n;
     plan->n_rank1 = n_rank1;
@@ -307,16 +321,31 @@ qf::Sched no_sched() {
     return sc;
 }
 
-unsigned panel_pre_grid(int64_t items) {   // one item per CTA and turn
-    return static_cast<unsigned>(std::min<int64_t>(items, static_cast<int64_t>(sm_count()) * qf::kPreMinCtas * kGridWaves));
+unsigned cta_grid(int64_t items, int per_sm) {   // one item per CTA and turn
+    return static_cast<unsigned>(std::min<int64_t>(items, static_cast<int64_t>(sm_count()) * per_sm * kGridWaves));
 }
 
 template <bool SCALE, bool SCHED>
 int launch_pre_panel(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
     const int dyn = qf::pre_dyn_smem(pl.any_f32_panel);
-    QF_CUDA(cudaFuncSetAttribute(qf::step_pre_kernel<true, SCALE, SCHED>, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::pre_dyn_smem(true)));
-    qf::step_pre_kernel<true, SCALE, SCHED><<<panel_pre_grid(pl.items[kPrePanel]), qf::kThreads, dyn, stream>>>(
+    QF_CUDA(cudaFuncSetAttribute(qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED>, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::pre_dyn_smem(true)));
+    qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED><<<cta_grid(pl.items[kPrePanel], qf::kPreMinCtas), qf::kThreads, dyn, stream>>>(
         pl.d_tensors, pl.d_base[kPrePanel], pl.n, hp, dyn / qf::kWarpsPerCta, pl.d_status, sc);
+    return QF_OK;
+}
+
+// First pass over the strips and over the flat items; the kernels see by themselves whether a gradient scale is set.
+template <bool SCHED>
+int launch_pre_others(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
+    if (pl.items[kStrip]) {
+        auto* kernel = qf::step_pre_kernel<qf::kMapStrip, false, SCHED>;
+        QF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::strip_dyn_smem()));
+        kernel<<<cta_grid(pl.items[kStrip], qf::kPreMinCtas), qf::kThreads, qf::strip_dyn_smem(), stream>>>(
+            pl.d_tensors, pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, sc);
+    }
+    if (pl.items[kPreFlat])
+        qf::step_pre_kernel<qf::kMapFlat, false, SCHED><<<persistent_grid(pl.items[kPreFlat], qf::kPreMinCtas), qf::kThreads, 0, stream>>>(
+            pl.d_tensors, pl.d_base[kPreFlat], pl.n, hp, 0, pl.d_status, sc);
     return QF_OK;
 }
 
@@ -338,15 +367,7 @@ int launch_pre(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStream
             rc = scaled ? launch_pre_panel<true, false>(pl, hp, no_sched(), stream) : launch_pre_panel<false, false>(pl, hp, no_sched(), stream);
         if (rc) return rc;
     }
-    if (pl.items[kPreFlat]) {
-        const unsigned grid = persistent_grid(pl.items[kPreFlat], qf::kPreMinCtas);
-        if (sched)
-            qf::step_pre_kernel<false, false, true><<<grid, qf::kThreads, 0, stream>>>(pl.d_tensors, pl.d_base[kPreFlat], pl.n, hp, 0,
-                                                                                     pl.d_status, *sched);
-        else
-            qf::step_pre_kernel<false><<<grid, qf::kThreads, 0, stream>>>(pl.d_tensors, pl.d_base[kPreFlat], pl.n, hp, 0, pl.d_status,
-                                                                          no_sched());
-    }
+    if (int rc = sched ? launch_pre_others<true>(pl, hp, *sched, stream) : launch_pre_others<false>(pl, hp, no_sched(), stream)) return rc;
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -355,9 +376,9 @@ template <bool PUSH, bool BC1, bool SCHED, bool RELAXED, int DT>
 int launch_main_panel_dt(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, cudaStream_t stream) {
     const int dyn = qf::main_dyn_smem(pl.any_f32_panel);
     const int ring = qf::kStages * (pl.any_f32_panel ? qf::kRowBytesF32 : qf::kRowBytesBf16);
-    QF_CUDA(cudaFuncSetAttribute(qf::step_main_kernel<true, PUSH, BC1, SCHED, RELAXED, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    QF_CUDA(cudaFuncSetAttribute(qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  qf::main_dyn_smem(true)));
-    qf::step_main_kernel<true, PUSH, BC1, SCHED, RELAXED, DT><<<persistent_grid(pl.items[kMainPanel], qf::kMainMinCtas), qf::kThreads, dyn, stream>>>(
+    qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT><<<persistent_grid(pl.items[kMainPanel], qf::kMainMinCtas), qf::kThreads, dyn, stream>>>(
         pl.d_tensors, pl.d_base[kMainPanel], pl.n, hp, ring, pl.d_status, pp, sc, pl.d_base[kRoll], static_cast<int>(pl.items[kRoll]));
     return QF_OK;
 }
@@ -373,8 +394,22 @@ int launch_main_panel(const Plan& pl, const qf::HyperPack& hp, const qf::PushPac
     return launch_main_panel_dt<PUSH, BC1, SCHED, RELAXED, 0>(pl, hp, pp, sc, stream);
 }
 
-// The new maxima are stored by the panel launch where there is one, else by the flat one.
-int flat_rolls(const Plan& pl) { return pl.items[kMainPanel] ? 0 : static_cast<int>(pl.items[kRoll]); }
+// Second pass over the strips and over the flat items.  The new maxima are stored by the first launch of the pass.
+template <bool PUSH, bool SCHED>
+int launch_main_others(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, cudaStream_t stream) {
+    int rolls = pl.items[kMainPanel] ? 0 : static_cast<int>(pl.items[kRoll]);
+    if (pl.items[kStrip]) {
+        auto* kernel = qf::step_main_kernel<qf::kMapStrip, PUSH, false, SCHED>;
+        QF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::strip_dyn_smem()));
+        kernel<<<cta_grid(pl.items[kStrip], qf::kMainMinCtas), qf::kThreads, qf::strip_dyn_smem(), stream>>>(
+            pl.d_tensors, pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls);
+        rolls = 0;
+    }
+    if (pl.items[kMainFlat])
+        qf::step_main_kernel<qf::kMapFlat, PUSH, false, SCHED><<<persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), qf::kThreads, 0, stream>>>(
+            pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls);
+    return QF_OK;
+}
 
 // bc_one: every hyper-parameter set of the call has bc2s == 1 exactly (late in a run): the panel kernel then
 // runs the variant without the division by it.
@@ -392,10 +427,7 @@ int launch_main_kernels(const Plan& pl, const qf::HyperPack& hp, const qf::PushP
                         : launch_main_panel<PUSH, false, false>(pl, hp, pp, no_sched(), stream);
         if (rc) return rc;
     }
-    if (pl.items[kMainFlat])
-        qf::step_main_kernel<false, PUSH><<<persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), qf::kThreads, 0, stream>>>(
-            pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, pp, no_sched(), pl.d_base[kRoll], flat_rolls(pl));
-    return QF_OK;
+    return launch_main_others<PUSH, false>(pl, hp, pp, no_sched(), stream);
 }
 
 // `push`: null, or the peer copies of the parameter buffer the kernels also store into.
@@ -413,9 +445,7 @@ int launch_main(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStrea
     if (sched) {
         if (pl.items[kMainPanel])
             if (int rc = launch_main_panel<false, false, true>(pl, hp, none, *sched, stream)) return rc;
-        if (pl.items[kMainFlat])
-            qf::step_main_kernel<false, false, false, true><<<persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), qf::kThreads, 0, stream>>>(
-                pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, none, *sched, pl.d_base[kRoll], flat_rolls(pl));
+        if (int rc = launch_main_others<false, true>(pl, hp, none, *sched, stream)) return rc;
     } else if (push && push->n > 0) {
         if (int rc = launch_main_kernels<true>(pl, hp, *push, bc_one, stream)) return rc;
     } else {
@@ -951,7 +981,11 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
         items = ceil_div(rows, t.main_rows) * t.panels;
         pre_items = ceil_div(rows, t.pre_rows * qf::kWarpsPerCta) * t.panels;
     }
-    const bool panel = t.flags & qf::kFlagPanel;
+    const bool panel = t.flags & qf::kFlagPanel, strip = !panel && strip_fits(cols, vec);
+    if (strip) {
+        t.flags |= qf::kFlagStrip;
+        t.strip_runs = strip_runs_for(ceil_div(t.numel, qf::strip_entries(qf::kStripRuns)));
+    }
 
     struct Header {
         uint32_t status[64];
@@ -962,9 +996,10 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     memset(&h, 0, sizeof h);
     h.t = t;
     h.base[kMainPanel][1] = panel ? items : 0;
-    h.base[kMainFlat][1] = panel ? 0 : items;
+    h.base[kMainFlat][1] = panel || strip ? 0 : items;
     h.base[kPrePanel][1] = panel ? pre_items : 0;
-    h.base[kPreFlat][1] = panel ? 0 : pre_items;
+    h.base[kPreFlat][1] = panel || strip ? 0 : pre_items;
+    h.base[kStrip][1] = strip ? ceil_div(t.numel, qf::strip_entries(t.strip_runs)) : 0;
     h.base[kRoll][1] = ceil_div(rows + cols, qf::kRollEntries);
     // The header goes up from this stack frame; a copy from pageable memory returns once the source has
     // been staged (for which the runtime may make the host wait for earlier work of the stream), so the frame

@@ -241,6 +241,26 @@ struct Raw8<__half> {
     }
 };
 
+// The first `nv` < 8 elements from e on, zeros behind them.
+template <typename T>
+__device__ __forceinline__ Raw8<T> raw8_tail(const char* base, int64_t e, int nv) {
+    union {
+        Raw8<T> raw;
+        uint32_t w[sizeof(T) * 2];
+    } u;
+#pragma unroll
+    for (int k = 0; k < static_cast<int>(sizeof(T)) * 2; ++k) u.w[k] = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (k >= nv) continue;
+        if (sizeof(T) == 4)
+            u.w[k % (sizeof(T) * 2)] = reinterpret_cast<const uint32_t*>(base)[e + k];
+        else
+            u.w[k / 2] |= static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(base)[e + k]) << (16 * (k & 1));
+    }
+    return u.raw;
+}
+
 __device__ __forceinline__ void load8f(const float* base, int64_t e, float (&x)[8]) {
     Elem<float>::load8(reinterpret_cast<const char*>(base), e, x);
 }

@@ -9,6 +9,9 @@
 //     the column only (old and new column maxima, their reciprocals) is fetched once per item (registers in
 //     the first pass, the warp's slice of shared memory in the main pass), and the first pass reduces column
 //     maxima over the rows in registers, then over the warps of the CTA, before touching global memory;
+//   * for the other rank-1 tensors (any column count from 8 on, vector-aligned buffers; "strip" mapping): runs of 256
+//     flattened elements like below, but dealt to whole CTAs, which keep the maxima of the columns that their strip of
+//     consecutive elements touches in shared memory;
 //   * otherwise ("flat" mapping): up to kRowsPerItem (16) consecutive runs of 256 flattened elements.
 // A multi-tensor launch numbers the work items of all tensors of one mapping consecutively; a warp finds
 // its tensor by binary search in the prefix-sum table.  The step kernels are persistent: CTAs of 8 warps,
@@ -59,12 +62,15 @@ struct DevTensor {
     int32_t main_rows;  // panel mapping: rows of one item of the second pass (kMainRowsPerItem, or fewer on small launches)
     int32_t pre_rows;   // panel mapping: rows of one item of the first pass (kPreRowsPerItem, or fewer on small launches)
     int32_t flat_runs;  // flat mapping: runs of 256 elements of one item (kRowsPerItem, or fewer on small launches)
-    int64_t pad1[2];
+    int32_t strip_runs; // strip mapping: runs of 256 elements per warp of one item
+    int32_t pad0;
+    int64_t pad1;
 };
 static_assert(sizeof(DevTensor) == 160, "DevTensor must stay 160 bytes");
 
 constexpr int kFlagVec = 1;    // every buffer is aligned for the vector path
 constexpr int kFlagPanel = 2;  // rank-1 tensor uses the panel mapping
+constexpr int kFlagStrip = 4;  // rank-1 tensor uses the strip mapping
 
 // Hyper-parameters as the kernels take them: the public scalars plus what the fast path needs.
 struct HyperDev {
@@ -363,9 +369,8 @@ __device__ __noinline__ uint32_t quantize8_pairs_exact(f2 a, f2 b, f2 c, f2 d, f
     return quantize8(x, scale, mid, 8);
 }
 
-// First-moment codes of a lane's 8 values against the block scale; fast division when the scale allows.
-__device__ __forceinline__ uint32_t quantize_m8(const f2 (&m)[4], float scale, const Smem& s) {
-    if (!scale_safe(scale)) return quantize8_pairs_exact(m[0], m[1], m[2], m[3], scale, s.t.mm);
+// First-moment codes of a lane's 8 values against a block scale that the division sequences may be used with.
+__device__ __forceinline__ uint32_t quantize_m8_safe(const f2 (&m)[4], float scale, const Smem& s) {
     const Recip rc = make_recip(scale);  // 0 for an all-zero block: every quotient is 0
     const f2 r2 = bc2(rc.r), ns2 = bc2(rc.nd);
     uint32_t w = 0;
@@ -376,6 +381,12 @@ __device__ __forceinline__ uint32_t quantize_m8(const f2 (&m)[4], float scale, c
         w += search_m_lut(q.y, s.mlut, s.t.mm) << (8 * j + 4);
     }
     return w;
+}
+
+// The same for any scale: fast division when it allows.
+__device__ __forceinline__ uint32_t quantize_m8(const f2 (&m)[4], float scale, const Smem& s) {
+    if (!scale_safe(scale)) return quantize8_pairs_exact(m[0], m[1], m[2], m[3], scale, s.t.mm);
+    return quantize_m8_safe(m, scale, s);
 }
 
 // Max of |x| over the 128-element block a lane's 8 values belong to (16 lanes), by redux instructions on the
@@ -1128,6 +1139,241 @@ __device__ __forceinline__ void main_flat(const DevTensor* tp, int64_t li, const
     }
 }
 
+// =================================================================================================
+// Strip mapping: rank-1 tensors whose rows are not whole panels
+// =================================================================================================
+//
+// An item is a strip of kThreads * 8 * strip_runs consecutive elements of the record, worked on by one CTA in runs of
+// 256 elements per warp; a lane's 8 elements lie in one row or cross into the next one (hence at least 8 columns).
+// The column scalars come from shared memory: entry i stands for column i where the strip covers all columns (the first
+// eight once more behind the last, so that a lane that crosses reads on), else -- a strip shorter than a row -- for the
+// i-th element of the strip.  Entries are spread by one word in 32, which makes a warp's accesses at a stride of 8 entries
+// conflict-free.  Column maxima are collected there as well and leave as one red.max per entry; row maxima by one redux
+// and red.max per run and row.  One atomic on the row and one on the column per element, as the flat mapping has it, costs
+// 3.4 ms for 20 M bf16 elements (50257 x 300, 3000 x 600, 1000 x 1500, ..), this 0.06 ms.
+constexpr int kStripRuns = 4;    // longest strip: 8192 elements
+__host__ __device__ constexpr int strip_entries(int runs) { return kThreads * 8 * runs; }
+__host__ __device__ constexpr int spread(int i) { return i + (i >> 5); }
+constexpr int kStripWords = spread(strip_entries(kStripRuns) + 8) + 1;
+constexpr int strip_dyn_smem() { return 2 * kStripWords * 4; }
+
+struct StripItem {
+    int64_t e0;       // first element of the strip inside the record
+    int entries;      // scalars in shared memory
+    int c_first;      // column of entry 0
+    int row_step, col_step;  // position of the element that lies one turn of the CTA (2048 elements) further on
+    bool window;      // the strip is shorter than a row: entry = element of the strip
+};
+// Row and column of element E of the matrix.
+__device__ __forceinline__ void position(int64_t E, int cols, int& r, int& c) {
+    if (E >> 32) {
+        r = static_cast<int>(E / cols);
+        c = static_cast<int>(E - static_cast<int64_t>(r) * cols);
+    } else {
+        const uint32_t q = static_cast<uint32_t>(E) / static_cast<uint32_t>(cols);
+        r = static_cast<int>(q);
+        c = static_cast<int>(static_cast<uint32_t>(E) - q * static_cast<uint32_t>(cols));
+    }
+}
+__device__ __forceinline__ StripItem strip_item(const DevTensor& t, int64_t li) {
+    StripItem o;
+    const int len = strip_entries(t.strip_runs);
+    o.e0 = li * len;
+    o.window = t.cols > len;
+    o.entries = o.window ? static_cast<int>(min(static_cast<int64_t>(len), t.numel - o.e0)) : t.cols + 8;
+    o.c_first = 0;
+    int r;
+    if (o.window) position(o.e0 + t.flat_off, t.cols, r, o.c_first);
+    o.row_step = (kThreads * 8) / t.cols;
+    o.col_step = (kThreads * 8) - o.row_step * t.cols;
+    return o;
+}
+__device__ __forceinline__ int strip_column(const StripItem& it, int i, int cols) {
+    const int c = it.c_first + i;
+    return c < cols ? c : c - cols;
+}
+// Word of the k-th of a lane's entries, for k known at compile time; `first` = the lane's first entry.
+__device__ __forceinline__ int strip_word(int first, int k) { return first + k + ((first + k) >> 5); }
+
+// The inputs of one run as loaded (zeros behind the end of the tensor).
+template <typename T>
+struct StripLoads {
+    Raw8<T> g;
+    uint32_t wv;
+    float row_a, row_b;
+};
+
+template <typename T>
+__device__ __forceinline__ void pre_strip(const DevTensor& t, int64_t li, const HyperDev& hd, const SmemPre& s, float* col_old,
+                                          uint32_t* col_max, uint32_t* status) {
+    const int lane = threadIdx.x & 31;
+    const StripItem it = strip_item(t, li);
+    const uint8_t* vc = reinterpret_cast<const uint8_t*>(t.v);
+    const Hyper2 h2 = widen(hd);
+    int off = static_cast<int>(threadIdx.x) * 8, r, c;   // this lane's first element of the strip
+    position(it.e0 + t.flat_off + off, t.cols, r, c);
+    auto load = [&](int off_, int r_) {
+        StripLoads<T> o;
+        const int64_t e = it.e0 + off_;
+        const int left = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(8), t.numel - e)));
+        if (left == 8) {
+            o.g.load(t.g, e);
+            o.wv = *reinterpret_cast<const uint32_t*>(vc + (e >> 1));
+        } else {
+            o.g = raw8_tail<T>(t.g, e, left);
+            o.wv = left ? load_codes_tail(vc, e, left) : 0u;
+        }
+        const int r_a = min(r_, t.rows - 1);
+        o.row_a = __ldg(t.vs + r_a);
+        o.row_b = __ldg(t.vs + min(r_a + 1, t.rows - 1));
+        return o;
+    };
+    StripLoads<T> next = load(off, r);     // the first run's inputs travel while the column scalars are fetched
+    for (int i = threadIdx.x; i < it.entries; i += kThreads) {
+        col_old[spread(i)] = __ldg(t.vcol + strip_column(it, i, t.cols));
+        col_max[spread(i)] = 0;
+    }
+    __syncthreads();
+    for (int run = 0; run < t.strip_runs; ++run) {
+        const int64_t e = it.e0 + off;
+        if (e - lane * 8 >= t.numel) break;   // warp-uniform
+        const StripLoads<T> now = next;
+        const int r_now = min(r, t.rows - 1), left = t.cols - c;   // elements from `left` on lie in the next row
+        const int first = it.window ? off : c;
+        const int nv = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(8), t.numel - e)));
+        off += kThreads * 8;
+        r += it.row_step;
+        c += it.col_step;
+        if (c >= t.cols) {
+            c -= t.cols;
+            ++r;
+        }
+        if (run + 1 < t.strip_runs) next = load(off, r);
+        float g[8];
+        now.g.widen(g);
+        if (hd.gs != 1.0f) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) g[k] = round_as<T>(__fmul_rn(g[k], hd.gs));
+            store8_masked<T>(const_cast<char*>(t.g), e, nv, true, g);
+        }
+        uint32_t max_a = 0, max_b = 0;
+        // an element behind the end of the tensor has gradient 0 and takes no part in the column maxima
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int w0 = strip_word(first, 2 * j), w1 = strip_word(first, 2 * j + 1);
+            const bool b0 = 2 * j >= left, b1 = 2 * j + 1 >= left;
+            const f2 scale = mk2(fminf(b0 ? now.row_b : now.row_a, col_old[w0]), fminf(b1 ? now.row_b : now.row_a, col_old[w1]));
+            const f2 v = v_update2(mk2(g[2 * j], g[2 * j + 1]), mul2(pair_lookup(s.qv2, now.wv, j), scale), h2);
+            const uint32_t x0 = 2 * j < nv ? __float_as_uint(v.x) : 0u, x1 = 2 * j + 1 < nv ? __float_as_uint(v.y) : 0u;
+            max_a = max(max_a, max(b0 ? 0u : x0, b1 ? 0u : x1));
+            max_b = max(max_b, max(b0 ? x0 : 0u, b1 ? x1 : 0u));
+            // mostly not a new maximum after the strip's first rows: look before the atomic
+            if (x0 > col_max[w0]) atomicMax(&col_max[w0], x0);
+            if (x1 > col_max[w1]) atomicMax(&col_max[w1], x1);
+        }
+        const int r_lo = __shfl_sync(kFull, r_now, 0);
+        const int r_hi = __reduce_max_sync(kFull, nv ? r_now + (nv > left ? 1 : 0) : 0);
+        for (int q = r_lo; q <= r_hi; ++q) {
+            const uint32_t m = __reduce_max_sync(kFull, max(r_now == q ? max_a : 0u, r_now + 1 == q ? max_b : 0u));
+            if (lane == 0) {
+                atomic_max_nonneg(t.vrow_new + q, m);
+                if (m >= 0x7f800000u) atomicOr(status, QF_STATUS_NONFINITE);
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < it.entries; i += kThreads) {
+        const uint32_t m = col_max[spread(i)];
+        if (m) atomic_max_nonneg(t.vcol_new + strip_column(it, i, t.cols), m);
+    }
+    __syncthreads();   // the next item fills the arrays again
+}
+
+// Second pass over a strip.  A full run takes the packed arithmetic -- with correctly rounded divisions for every dtype,
+// as the exact path has them -- where its scalars allow it (old and new maxima of its rows and of the strip's columns in
+// [2^-80, 2^100], the old first-moment scale finite, the new one zero or in range); any other run goes through
+// main_flat_run_exact.  Nothing of a run is stored before that is known.
+__device__ __forceinline__ bool strip_scale_ok(float x) { return x >= 0x1p-80f && x <= 0x1p100f; }
+template <typename T, bool PUSH>
+__device__ __forceinline__ void main_strip(const DevTensor* tp, int64_t li, const HyperDev& hd, const Smem& s, float* col_old,
+                                           float* col_new, uint32_t* status, const PushPack* push) {
+    const DevTensor t = *tp;
+    const int lane = threadIdx.x & 31;
+    const StripItem it = strip_item(t, li);
+    bool fit = hd.fast;
+    for (int i = threadIdx.x; i < it.entries; i += kThreads) {
+        const int c = strip_column(it, i, t.cols);
+        const float old = __ldg(t.vcol_old + c), fresh = __ldg(t.vcol_new + c);
+        fit &= strip_scale_ok(old) && strip_scale_ok(fresh);
+        col_old[spread(i)] = old;
+        col_new[spread(i)] = fresh;
+    }
+    const bool cols_fit = __syncthreads_and(fit);
+    uint8_t* mc = reinterpret_cast<uint8_t*>(t.m);
+    uint8_t* vc = reinterpret_cast<uint8_t*>(t.v);
+    const Hyper2 h2 = widen(hd);
+    int off = static_cast<int>(threadIdx.x) * 8, r, c;
+    position(it.e0 + t.flat_off + off, t.cols, r, c);
+    for (int run = 0; run < t.strip_runs; ++run) {
+        const int64_t e = it.e0 + off, wbase = e - lane * 8;
+        if (wbase >= t.numel) break;   // warp-uniform
+        bool done = false;
+        if (cols_fit && wbase + kPanelCols <= t.numel) {
+            Raw8<T> p_raw, g_raw;
+            p_raw.load(t.p, e);
+            g_raw.load(t.g, e);
+            const uint32_t wm = *reinterpret_cast<const uint32_t*>(mc + (e >> 1));
+            const uint32_t wv = *reinterpret_cast<const uint32_t*>(vc + (e >> 1));
+            const float ms = __ldg(t.ms + (e >> 7));
+            const int left = t.cols - c, r_b = min(r + 1, t.rows - 1), first = it.window ? off : c;
+            const float old_a = __ldg(t.vrow_old + r), old_b = __ldg(t.vrow_old + r_b);
+            const float new_a = __ldg(t.vrow_new + r), new_b = __ldg(t.vrow_new + r_b);
+            bool ok = strip_scale_ok(old_a) && strip_scale_ok(new_a) && ms < __builtin_huge_valf();
+            ok = ok && (left >= 8 || (strip_scale_ok(old_b) && strip_scale_ok(new_b)));
+            float p[8], g[8];
+            p_raw.widen(p);
+            g_raw.widen(g);
+            f2 m[4];
+            int cv[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int w0 = strip_word(first, 2 * j), w1 = strip_word(first, 2 * j + 1);
+                const bool b0 = 2 * j >= left, b1 = 2 * j + 1 >= left;
+                const f2 so = mk2(fminf(b0 ? old_b : old_a, col_old[w0]), fminf(b1 ? old_b : old_a, col_old[w1]));
+                const f2 sn = mk2(fminf(b0 ? new_b : new_a, col_new[w0]), fminf(b1 ? new_b : new_a, col_new[w1]));
+                f2 pp = mk2(p[2 * j], p[2 * j + 1]);
+                f2 v = mul2(pair_entry(s.qv2, wv, j), so);
+                m[j] = mul2(pair_entry(s.qm2, wm, j), bc2(ms));
+                adamw_pair<true>(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v, h2);
+                p[2 * j] = pp.x;
+                p[2 * j + 1] = pp.y;
+                const f2 y = fma2(div2(v, sn), bc2(16.0f), bc2(-1.5f));
+                cv[2 * j] = ceil_s32(y.x);       // at most 15: the scale is a maximum over values that include v
+                cv[2 * j + 1] = ceil_s32(y.y);
+            }
+            const float ms_new = absmax_pairs_to_block_nan(m);
+            if (__all_sync(kFull, ok && scale_safe(ms_new))) {
+                Elem<T>::store8(t.p, e, p);
+                if (PUSH) push_store8<T>(t.p, e, p, push);
+                *reinterpret_cast<uint32_t*>(mc + (e >> 1)) = quantize_m8_safe(m, ms_new, s);
+                *reinterpret_cast<uint32_t*>(vc + (e >> 1)) =
+                    pack_u4(cv[1], cv[0], pack_u4(cv[3], cv[2], pack_u4(cv[5], cv[4], pack_u4(cv[7], cv[6], 0u))));
+                if ((lane & 15) == 0) t.ms[e >> 7] = ms_new;
+                done = true;
+            }
+        }
+        if (!done) main_flat_run_exact<T, QF_KIND_RANK1>(tp, wbase, hd, s, status, PUSH ? push : nullptr);
+        off += kThreads * 8;
+        r += it.row_step;
+        c += it.col_step;
+        if (c >= t.cols) {
+            c -= t.cols;
+            ++r;
+        }
+    }
+    __syncthreads();   // the next item fills the arrays again
+}
+
 // Small passes over the row / column maxima of every rank-1 tensor, as bits of `mode`:
 //   kRollClear     new maxima := 0                        (before the first pass)
 //   kRollKeep      copy of the stored maxima for the second pass
@@ -1167,11 +1413,12 @@ rank1_roll_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restri
 
 // The multi-tensor kernels are persistent: the host launches about as many CTAs as fit on the device and every
 // warp walks the item list with a fixed stride, so the shared-memory tables are filled once per CTA.
+enum { kMapFlat = 0, kMapPanel = 1, kMapStrip = 2 };   // MAP: the mapping a kernel serves
 constexpr int kPreMinCtas = 3;   // CTAs per SM the first pass is compiled for (80 registers)
 // SCALE (panel mapping): some hyper-parameter set of the launch carries a gradient scale other than 1.
 // SCHED: the hyper-parameter sets come from the device-resident table `sc` instead of `hp`.
 // (Forms of this kernel that carry one dtype's loop only, as step_main_kernel has them, measured 5 % slower.)
-template <bool PANEL, bool SCALE = false, bool SCHED = false>
+template <int MAP, bool SCALE = false, bool SCHED = false>
 __global__ void __launch_bounds__(kThreads, kPreMinCtas)
 step_pre_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict__ base, int n,
                 const __grid_constant__ HyperPack hp, int ring_bytes, uint32_t* status, const __grid_constant__ Sched sc) {
@@ -1181,13 +1428,22 @@ step_pre_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict
     load_smem(s);
     extern __shared__ __align__(16) char staging[];  // panel kernel: one ring of rows per warp
     char* stage = staging + (threadIdx.x >> 5) * ring_bytes;
-    const int64_t total = base[n], per_cta = PANEL ? 1 : kWarpsPerCta, stride = gridDim.x * per_cta;
-    for (int64_t item = blockIdx.x * per_cta + (PANEL ? 0 : threadIdx.x >> 5); item < total; item += stride) {
+    const int64_t total = base[n], per_cta = MAP == kMapFlat ? kWarpsPerCta : 1, stride = gridDim.x * per_cta;
+    for (int64_t item = blockIdx.x * per_cta + (MAP == kMapFlat ? threadIdx.x >> 5 : 0); item < total; item += stride) {
         const int ti = find_tensor(base, n, item);
         const DevTensor t = tensors[ti];
         const int64_t li = item - base[ti];
         const HyperDev& h = SCHED ? sched_h[t.hyper] : hp.h[t.hyper];
-        if (PANEL) {
+        if (MAP == kMapStrip) {
+            float* words = reinterpret_cast<float*>(staging);
+            uint32_t* col_max = reinterpret_cast<uint32_t*>(words + kStripWords);
+            if (t.dtype == QF_BF16)
+                pre_strip<__nv_bfloat16>(t, li, h, s, words, col_max, status);
+            else if (t.dtype == QF_F16)
+                pre_strip<__half>(t, li, h, s, words, col_max, status);
+            else
+                pre_strip<float>(t, li, h, s, words, col_max, status);
+        } else if (MAP == kMapPanel) {
             if (t.dtype == QF_BF16)
                 pre_panel<__nv_bfloat16, SCALE>(t, li, h, s, stage, ring_bytes, status);
             else if (t.dtype == QF_F16)
@@ -1226,7 +1482,7 @@ constexpr int kMainMinCtas = 2;  // CTAs per SM the second pass is compiled for 
 // only; a kernel that carries one dtype's loop is scheduled a little better than one that carries all.
 // Every CTA ends with its share of the `n_roll` items that store the new row / column maxima (kRollCommit): the second
 // pass reads the old ones from the copies, so nothing has to wait for them.
-template <bool PANEL, bool PUSH, bool BC1 = false, bool SCHED = false, bool RELAXED = false, int DT = 0>
+template <int MAP, bool PUSH, bool BC1 = false, bool SCHED = false, bool RELAXED = false, int DT = 0>
 __global__ void __launch_bounds__(kThreads, kMainMinCtas)
 step_main_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict__ base, int n,
                  const __grid_constant__ HyperPack hp, int ring_bytes, uint32_t* status,
@@ -1238,13 +1494,21 @@ step_main_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restric
     load_smem(s);
     extern __shared__ __align__(16) char staging[];  // panel kernel: per warp a ring of rows plus the column block
     char* stage = staging + (threadIdx.x >> 5) * (ring_bytes + kColBytes + kRowBufBytes);
-    const int64_t total = base[n], stride = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
-    for (int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5); item < total; item += stride) {
+    const int64_t total = base[n], per_cta = MAP == kMapStrip ? 1 : kWarpsPerCta, stride = gridDim.x * per_cta;
+    for (int64_t item = blockIdx.x * per_cta + (MAP == kMapStrip ? 0 : threadIdx.x >> 5); item < total; item += stride) {
         const int ti = find_tensor(base, n, item);
         const DevTensor* tp = tensors + ti;
         const int64_t li = item - base[ti];
         const HyperDev& h = SCHED ? sched_h[tp->hyper] : hp.h[tp->hyper];  // hp is a grid constant: its address is usable as it is
-        if (PANEL) {
+        if (MAP == kMapStrip) {
+            float* words = reinterpret_cast<float*>(staging);
+            if (tp->dtype == QF_BF16)
+                main_strip<__nv_bfloat16, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
+            else if (tp->dtype == QF_F16)
+                main_strip<__half, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
+            else
+                main_strip<float, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
+        } else if (MAP == kMapPanel) {
             if (DT == 1 || (DT == 0 && tp->dtype == QF_BF16))
                 main_panel<__nv_bfloat16, PUSH, BC1, RELAXED>(tp, li, h, s, stage, ring_bytes, status, push);
             else if (DT == 3 || (DT == 0 && tp->dtype == QF_F16))

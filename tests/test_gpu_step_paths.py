@@ -53,3 +53,15 @@ def test_panels_of_several_dtypes_in_one_launch():
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_rows_without_state_and_gradient(dtype):
     run([((130, 512), dtype), ((257, 256), dtype)], dead_rows=0.5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(5000, 1), (1000, 7), (1000, 8), (1001, 9), (600, 77), (100, 255), (65, 257), (31, 2047), (31, 2049),
+                                   (9, 8191), (9, 8193), (5, 20001), (1, 9000)])
+def test_matrices_whose_rows_are_no_whole_panels(shape, dtype):
+    run([(shape, dtype)], steps=3)
+
+
+def test_strips_flat_items_and_panels_in_one_launch():
+    run([((300, 300), torch.bfloat16), ((500,), torch.bfloat16), ((64, 512), torch.bfloat16), ((77, 333), torch.float16),
+         ((9001,), torch.float32), ((1200, 1500), torch.float32)], dead_rows=0.2)
