@@ -107,23 +107,36 @@ struct Plan {
 };
 
 int sm_count();
-// Length of a work item (rows of a panel, runs of the flat mapping): the longest of longest, longest / 2, .. shortest
-// that still gives every slot of the device (`per_sm` per SM) one; `items` = the number of items of the longest form.
-int item_length(int64_t items, int longest, int shortest, int per_sm) {
+// Length of a work item (rows of a panel, runs of the flat mapping or of a strip).  `units` rows or runs in all, shared out
+// among `slots` warps or CTAs; an item costs its length plus `fixed`.  Taken is the length, a multiple of `step` in
+// [shortest, longest], whose rounds of the device cost least: as long as possible while every slot has an item and the
+// last round is full (28 rows instead of 16 for a 4096 x 4096 matrix: one round instead of 1.7; 56 instead of 64 rows for
+// the 202 M elements of a 7B decoder layer: 6.0 rounds instead of 5.2).
+int item_length(int64_t units, int longest, int shortest, int step, int fixed, int per_sm) {
     const int64_t slots = static_cast<int64_t>(sm_count()) * per_sm;
-    int len = longest;
-    while (len > shortest && items * (longest / len) < slots) len /= 2;
-    return len;
+    int best = longest;
+    int64_t best_cost = INT64_MAX;
+    for (int len = longest; len >= shortest; len -= step) {
+        const int64_t cost = ceil_div(ceil_div(units, len), slots) * (len + fixed);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = len;
+        }
+    }
+    return best;
 }
-int main_rows_for(int64_t items) {
-    return item_length(items, qf::kMainRowsPerItem, qf::kMinMainRowsPerItem, qf::kMainMinCtas * qf::kWarpsPerCta);
+int main_rows_for(int64_t rows) {
+    return item_length(rows, qf::kMainRowsPerItem, qf::kMinMainRowsPerItem, 2, 2, qf::kMainMinCtas * qf::kWarpsPerCta);
 }
-// two CTA items per slot: 512 rows per item left the device a ragged last wave (202 M elements: 139 -> 125 us)
-int pre_rows_for(int64_t items) { return item_length(items, qf::kPreRowsPerItem, qf::kMinPreRowsPerItem, 2 * qf::kPreMinCtas); }
-int flat_runs_for(int64_t items) { return item_length(items, qf::kRowsPerItem, qf::kMinRowsPerItem, qf::kMainMinCtas * qf::kWarpsPerCta); }
+int pre_rows_for(int64_t rows) {   // rows per warp of a CTA's item
+    return item_length(ceil_div(rows, qf::kWarpsPerCta), qf::kPreRowsPerItem, qf::kMinPreRowsPerItem, 8, 4, qf::kPreMinCtas);
+}
+int flat_runs_for(int64_t runs) {
+    return item_length(runs, qf::kRowsPerItem, qf::kMinRowsPerItem, 1, 1, qf::kMainMinCtas * qf::kWarpsPerCta);
+}
+int strip_runs_for(int64_t runs) { return item_length(ceil_div(runs, qf::kWarpsPerCta), qf::kStripRuns, 1, 1, 1, qf::kMainMinCtas); }
+int64_t runs_of(int64_t numel) { return ceil_div(numel, qf::kPanelCols); }
 
-// Strips: two CTAs' worth per SM of the shortest length, as for the other mappings.
-int strip_runs_for(int64_t items) { return item_length(items, qf::kStripRuns, 1, qf::kMainMinCtas); }
 // The strip mapping takes a rank-1 tensor that is not whole panels if its buffers are vector-aligned and a lane's eight
 // elements cross at most one row end.
 bool strip_fits(int64_t cols, bool vec) { return vec && cols >= 8; }
@@ -144,6 +157,7 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
     for (auto& b : base) b.push_back(0);
     tab.reserve(n_tensors);
     int n_rank1 = 0;
+    int64_t panel_rows = 0, strip_runs_all = 0, flat_runs_all = 0;   // rows of 256 columns, runs of 256 elements
     for (int i = 0; i < n_tensors; ++i) {
         const QfTensorDesc& d = descs[i];
         if (d.numel < 0) return fail(QF_ERR_BAD_ARG, "tensor %d: negative numel", i);
@@ -175,7 +189,6 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
             t.ms = d.m_scale;
             t.vs = d.v_scale;
         }
-        int64_t items = flat_items(d.numel), pre_items = items;
         if (d.kind == QF_KIND_RANK1) {
             if (d.rows <= 0 || d.cols <= 0 || d.rows > INT32_MAX || d.cols > INT32_MAX || d.flat_offset < 0 ||
                 d.flat_offset + d.numel > d.rows * d.cols || (d.flat_offset == 0 && !d.partial && d.rows * d.cols != d.numel))
@@ -199,8 +212,6 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
             if (panel) {
                 t.flags |= qf::kFlagPanel;
                 t.panels = static_cast<int32_t>(d.cols / qf::kPanelCols);
-                items = (d.rows + qf::kMainRowsPerItem - 1) / qf::kMainRowsPerItem * t.panels;
-                pre_items = ceil_div(d.rows, qf::kPreRowsPerItem * qf::kWarpsPerCta) * t.panels;
                 if (d.dtype == QF_F32) plan->any_f32_panel = true;
                 if (d.dtype == QF_BF16) plan->any_bf16_panel = true;
                 if (d.dtype == QF_F16) plan->any_f16_panel = true;
@@ -210,20 +221,16 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
             ++n_rank1;
         }
         if (vec) t.flags |= qf::kFlagVec;
-        const bool panel = t.flags & qf::kFlagPanel, strip = t.flags & qf::kFlagStrip, rank1 = d.kind == QF_KIND_RANK1;
-        // items of the longest form; shorter ones are chosen below from these sums
-        base[kMainPanel].push_back(base[kMainPanel].back() + (panel ? items : 0));
-        base[kMainFlat].push_back(base[kMainFlat].back() + (panel || strip ? 0 : items));
-        base[kPrePanel].push_back(base[kPrePanel].back() + (panel ? pre_items : 0));
-        base[kPreFlat].push_back(0);
-        base[kRoll].push_back(base[kRoll].back() + (rank1 ? ceil_div(d.rows + d.cols, qf::kRollEntries) : 0));
-        base[kStrip].push_back(base[kStrip].back() + (strip ? ceil_div(d.numel, qf::strip_entries(qf::kStripRuns)) : 0));
+        const bool panel = t.flags & qf::kFlagPanel, strip = t.flags & qf::kFlagStrip;
+        if (panel)
+            panel_rows += d.rows * t.panels;
+        else
+            (strip ? strip_runs_all : flat_runs_all) += runs_of(d.numel);
         tab.push_back(t);
     }
     const int n = static_cast<int>(tab.size());
-    // a small launch: shorter items, so that the whole device takes part
-    const int main_rows = main_rows_for(base[kMainPanel].back()), pre_rows = pre_rows_for(base[kPrePanel].back());
-    const int flat_runs = flat_runs_for(base[kMainFlat].back()), strip_runs = strip_runs_for(base[kStrip].back());
+    const int main_rows = main_rows_for(panel_rows), pre_rows = pre_rows_for(panel_rows);
+    const int flat_runs = flat_runs_for(flat_runs_all), strip_runs = strip_runs_for(strip_runs_all);
     int64_t acc[kTables] = {};
     for (int i = 0; i < n; ++i) {
         qf::DevTensor& t = tab[i];
@@ -241,8 +248,8 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
             acc[kMainFlat] += items;
             if (t.kind == QF_KIND_RANK1) acc[kPreFlat] += items;
         }
-        acc[kRoll] = base[kRoll][i + 1];
-        for (int k = 0; k < kTables; ++k) base[k][i + 1] = acc[k];
+        if (t.kind == QF_KIND_RANK1) acc[kRoll] += ceil_div(static_cast<int64_t>(t.rows) + t.cols, qf::kRollEntries);
+        for (int k = 0; k < kTables; ++k) base[k].push_back(acc[k]);
     }
     plan->n = n;
     plan->n_rank1 = n_rank1;
@@ -311,8 +318,26 @@ unsigned persistent_grid(int64_t items, int per_sm, int waves = kGridWaves) {
     return static_cast<unsigned>(ctas < cap ? ctas : cap);
 }
 
-void roll(const Plan& pl, int mode, cudaStream_t stream) {
-    qf::rank1_roll_kernel<<<static_cast<unsigned>(pl.items[kRoll]), qf::kThreads, 0, stream>>>(pl.d_tensors, pl.d_base[kRoll], pl.n, mode);
+// A kernel of a step, launched so that it may be set up while the kernel ahead of it on the stream drains (every such
+// kernel waits for that one's end before it touches memory: dependency_wait in qf_device.cuh).
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(qf::kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+int roll(const Plan& pl, int mode, cudaStream_t stream) {
+    QF_CUDA(launch_chained(qf::rank1_roll_kernel, static_cast<unsigned>(pl.items[kRoll]), 0, stream, pl.d_tensors, pl.d_base[kRoll], pl.n, mode));
+    return QF_OK;
 }
 
 qf::Sched no_sched() {
@@ -329,8 +354,8 @@ template <bool SCALE, bool SCHED>
 int launch_pre_panel(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
     const int dyn = qf::pre_dyn_smem(pl.any_f32_panel);
     QF_CUDA(cudaFuncSetAttribute(qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED>, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::pre_dyn_smem(true)));
-    qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED><<<cta_grid(pl.items[kPrePanel], qf::kPreMinCtas), qf::kThreads, dyn, stream>>>(
-        pl.d_tensors, pl.d_base[kPrePanel], pl.n, hp, dyn / qf::kWarpsPerCta, pl.d_status, sc);
+    QF_CUDA(launch_chained(qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED>, cta_grid(pl.items[kPrePanel], qf::kPreMinCtas), dyn, stream,
+                           pl.d_tensors, pl.d_base[kPrePanel], pl.n, hp, dyn / qf::kWarpsPerCta, pl.d_status, sc));
     return QF_OK;
 }
 
@@ -340,12 +365,11 @@ int launch_pre_others(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& 
     if (pl.items[kStrip]) {
         auto* kernel = qf::step_pre_kernel<qf::kMapStrip, false, SCHED>;
         QF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::strip_dyn_smem()));
-        kernel<<<cta_grid(pl.items[kStrip], qf::kPreMinCtas), qf::kThreads, qf::strip_dyn_smem(), stream>>>(
-            pl.d_tensors, pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, sc);
+        QF_CUDA(launch_chained(kernel, cta_grid(pl.items[kStrip], qf::kPreMinCtas), qf::strip_dyn_smem(), stream, pl.d_tensors, pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, sc));
     }
     if (pl.items[kPreFlat])
-        qf::step_pre_kernel<qf::kMapFlat, false, SCHED><<<persistent_grid(pl.items[kPreFlat], qf::kPreMinCtas), qf::kThreads, 0, stream>>>(
-            pl.d_tensors, pl.d_base[kPreFlat], pl.n, hp, 0, pl.d_status, sc);
+        QF_CUDA(launch_chained(qf::step_pre_kernel<qf::kMapFlat, false, SCHED>, persistent_grid(pl.items[kPreFlat], qf::kPreMinCtas), 0, stream,
+                               pl.d_tensors, pl.d_base[kPreFlat], pl.n, hp, 0, pl.d_status, sc));
     return QF_OK;
 }
 
@@ -355,7 +379,7 @@ int launch_pre_others(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& 
 int launch_pre(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStream_t stream, bool keep, const qf::Sched* sched = nullptr,
                bool scaled = false) {
     if (pl.n_rank1 == 0) return QF_OK;
-    roll(pl, qf::kRollClear | (keep ? qf::kRollKeep : 0), stream);
+    if (int rc = roll(pl, qf::kRollClear | (keep ? qf::kRollKeep : 0), stream)) return rc;
     if (pl.items[kPrePanel]) {
         // the variant that rewrites the gradients runs only when some set asks for it
         if (!sched)
@@ -378,8 +402,8 @@ int launch_main_panel_dt(const Plan& pl, const qf::HyperPack& hp, const qf::Push
     const int ring = qf::kStages * (pl.any_f32_panel ? qf::kRowBytesF32 : qf::kRowBytesBf16);
     QF_CUDA(cudaFuncSetAttribute(qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  qf::main_dyn_smem(true)));
-    qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT><<<persistent_grid(pl.items[kMainPanel], qf::kMainMinCtas), qf::kThreads, dyn, stream>>>(
-        pl.d_tensors, pl.d_base[kMainPanel], pl.n, hp, ring, pl.d_status, pp, sc, pl.d_base[kRoll], static_cast<int>(pl.items[kRoll]));
+    QF_CUDA(launch_chained(qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT>, persistent_grid(pl.items[kMainPanel], qf::kMainMinCtas), dyn, stream,
+                           pl.d_tensors, pl.d_base[kMainPanel], pl.n, hp, ring, pl.d_status, pp, sc, pl.d_base[kRoll], static_cast<int>(pl.items[kRoll])));
     return QF_OK;
 }
 // A launch whose panel tensors are all of one dtype takes the kernel that carries that dtype's loop only (the plain
@@ -401,13 +425,12 @@ int launch_main_others(const Plan& pl, const qf::HyperPack& hp, const qf::PushPa
     if (pl.items[kStrip]) {
         auto* kernel = qf::step_main_kernel<qf::kMapStrip, PUSH, false, SCHED>;
         QF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::strip_dyn_smem()));
-        kernel<<<cta_grid(pl.items[kStrip], qf::kMainMinCtas), qf::kThreads, qf::strip_dyn_smem(), stream>>>(
-            pl.d_tensors, pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls);
+        QF_CUDA(launch_chained(kernel, cta_grid(pl.items[kStrip], qf::kMainMinCtas), qf::strip_dyn_smem(), stream, pl.d_tensors, pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls));
         rolls = 0;
     }
     if (pl.items[kMainFlat])
-        qf::step_main_kernel<qf::kMapFlat, PUSH, false, SCHED><<<persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), qf::kThreads, 0, stream>>>(
-            pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls);
+        QF_CUDA(launch_chained(qf::step_main_kernel<qf::kMapFlat, PUSH, false, SCHED>, persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), 0, stream,
+                               pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls));
     return QF_OK;
 }
 
@@ -437,7 +460,8 @@ int launch_main_kernels(const Plan& pl, const qf::HyperPack& hp, const qf::PushP
 int launch_main(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStream_t stream, bool kept, const qf::PushPack* push = nullptr,
                 const qf::Sched* sched = nullptr, bool relaxed = false) {
     if (pl.n == 0) return QF_OK;
-    if (pl.n_rank1 && !kept) roll(pl, qf::kRollKeep, stream);
+    if (pl.n_rank1 && !kept)
+        if (int rc = roll(pl, qf::kRollKeep, stream)) return rc;
     bool bc_one = true;
     for (int k = 0; k < n_hypers; ++k) bc_one = bc_one && hp.h[k].fast && hp.h[k].h.bc2s == 1.0f;
     qf::PushPack none;
@@ -769,13 +793,13 @@ int qf_fused_4bit(void* p, const void* g, void* exp, void* sq, float* exp_scale,
     t.vs = sq_scale;
     t.numel = numel;
     t.kind = QF_KIND_BLOCK;
-    t.flat_runs = flat_runs_for(flat_items(numel));
+    t.flat_runs = flat_runs_for(runs_of(numel));
     t.dtype = dtype;
     if (aligned(p, 16) && aligned(g, 16) && aligned(exp, 4) && aligned(sq, 4)) t.flags |= qf::kFlagVec;
     QfHyper h;
     qf_make_hyper(lr, beta1, beta2, eps, weight_decay, step, &h);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    qf::single_tensor_kernel<<<single_grid(t), qf::kThreads, 0, st>>>(t, widen_hyper(h));
+    QF_CUDA(launch_chained(qf::single_tensor_kernel, single_grid(t), 0, st, t, widen_hyper(h)));
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -799,13 +823,13 @@ int qf_fused_single_tensor(void* p, const void* g, float* exp_avg, float* exp_av
     t.v = reinterpret_cast<char*>(exp_avg_sq);
     t.numel = numel;
     t.kind = QF_KIND_FP32;
-    t.flat_runs = flat_runs_for(flat_items(numel));
+    t.flat_runs = flat_runs_for(runs_of(numel));
     t.dtype = dtype;
     if (aligned(p, 16) && aligned(g, 16) && aligned(exp_avg, 16) && aligned(exp_avg_sq, 16)) t.flags |= qf::kFlagVec;
     QfHyper h;
     qf_make_hyper(lr, beta1, beta2, eps, weight_decay, step, &h);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    qf::single_tensor_kernel<<<single_grid(t), qf::kThreads, 0, st>>>(t, widen_hyper(h));
+    QF_CUDA(launch_chained(qf::single_tensor_kernel, single_grid(t), 0, st, t, widen_hyper(h)));
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -971,20 +995,20 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     t.dtype = dtype;
     const bool vec = aligned(p, 16) && aligned(g, 16) && aligned(m_codes, 4) && aligned(v_codes, 4);
     if (vec) t.flags |= qf::kFlagVec;
-    t.flat_runs = flat_runs_for(flat_items(t.numel));
+    t.flat_runs = flat_runs_for(runs_of(t.numel));
     int64_t items = ceil_div(t.numel, static_cast<int64_t>(qf::kPanelCols) * t.flat_runs), pre_items = items;
     if (vec && t.numel < (1ll << 31) && cols % qf::kPanelCols == 0 && aligned(v_col, 16)) {
         t.flags |= qf::kFlagPanel;
         t.panels = static_cast<int32_t>(cols / qf::kPanelCols);
-        t.main_rows = main_rows_for(ceil_div(rows, qf::kMainRowsPerItem) * t.panels);
-        t.pre_rows = pre_rows_for(ceil_div(rows, qf::kPreRowsPerItem * qf::kWarpsPerCta) * t.panels);
+        t.main_rows = main_rows_for(rows * t.panels);
+        t.pre_rows = pre_rows_for(rows * t.panels);
         items = ceil_div(rows, t.main_rows) * t.panels;
         pre_items = ceil_div(rows, t.pre_rows * qf::kWarpsPerCta) * t.panels;
     }
     const bool panel = t.flags & qf::kFlagPanel, strip = !panel && strip_fits(cols, vec);
     if (strip) {
         t.flags |= qf::kFlagStrip;
-        t.strip_runs = strip_runs_for(ceil_div(t.numel, qf::strip_entries(qf::kStripRuns)));
+        t.strip_runs = strip_runs_for(runs_of(t.numel));
     }
 
     struct Header {

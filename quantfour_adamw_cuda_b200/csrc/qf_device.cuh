@@ -44,32 +44,34 @@ constexpr unsigned kFull = 0xffffffffu;
 // Code books.  Literals as in optim/cuda_adamw_kernels.cu:25-98 (= optim/adamw_fourbit_triton.py:16-97):
 // decimal constants rounded once to fp32.  The midpoint tables are the reference's own literals, not
 // recomputed from the maps (they differ by one ulp at +-0.145).
-__device__ __constant__ float c_qm[16] = {-0.8875f, -0.6625f, -0.4375f, -0.2125f, -0.0775f, -0.0325f,
-                                          -0.0055f, 0.0f,     0.0055f,  0.0325f,  0.0775f,  0.2125f,
-                                          0.4375f,  0.6625f,  0.8875f,  1.0f};
-__device__ __constant__ float c_mm[16] = {-0.775f, -0.55f, -0.325f, -0.145f, -0.055f, -0.019f, -0.00275f, 0.00275f,
-                                          0.019f,  0.055f, 0.145f,  0.325f,  0.55f,   0.775f,  0.94375f,
-                                          __builtin_huge_valf()};
-__device__ __constant__ float c_qv[16] = {0.0625f, 0.125f, 0.1875f, 0.25f, 0.3125f, 0.375f, 0.4375f, 0.5f,
-                                          0.5625f, 0.625f, 0.6875f, 0.75f, 0.8125f, 0.875f, 0.9375f, 1.0f};
-__device__ __constant__ float c_mv[16] = {0.09375f, 0.15625f, 0.21875f, 0.28125f, 0.34375f, 0.40625f,
-                                          0.46875f, 0.53125f, 0.59375f, 0.65625f, 0.71875f, 0.78125f,
-                                          0.84375f, 0.90625f, 0.96875f, __builtin_huge_valf()};
+constexpr float kQm[16] = {-0.8875f, -0.6625f, -0.4375f, -0.2125f, -0.0775f, -0.0325f, -0.0055f, 0.0f,
+                           0.0055f, 0.0325f, 0.0775f, 0.2125f, 0.4375f, 0.6625f, 0.8875f, 1.0f};
+constexpr float kMm[16] = {-0.775f, -0.55f, -0.325f, -0.145f, -0.055f, -0.019f, -0.00275f, 0.00275f,
+                           0.019f, 0.055f, 0.145f, 0.325f, 0.55f, 0.775f, 0.94375f, __builtin_huge_valf()};
+constexpr float kQv[16] = {0.0625f, 0.125f, 0.1875f, 0.25f, 0.3125f, 0.375f, 0.4375f, 0.5f,
+                           0.5625f, 0.625f, 0.6875f, 0.75f, 0.8125f, 0.875f, 0.9375f, 1.0f};
+constexpr float kMv[16] = {0.09375f, 0.15625f, 0.21875f, 0.28125f, 0.34375f, 0.40625f, 0.46875f, 0.53125f,
+                           0.59375f, 0.65625f, 0.71875f, 0.78125f, 0.84375f, 0.90625f, 0.96875f, __builtin_huge_valf()};
 
-// Shared-memory copy of the tables, one per CTA.
+// The tables as every CTA keeps them in shared memory.
 struct Tables {
     float qm[16], mm[16], qv[16], mv[16];
 };
 
-__device__ __forceinline__ void load_tables(Tables& s) {
-    if (threadIdx.x < 16) {
-        s.qm[threadIdx.x] = c_qm[threadIdx.x];
-        s.mm[threadIdx.x] = c_mm[threadIdx.x];
-        s.qv[threadIdx.x] = c_qv[threadIdx.x];
-        s.mv[threadIdx.x] = c_mv[threadIdx.x];
-    }
-    __syncthreads();
+// Copies a table that the compiler has laid out in device memory into shared memory, 16 bytes per thread and turn.  (The
+// pair tables computed by every CTA from the 16-entry ones in constant memory, whose index differs by lane, cost up to 16
+// constant loads one after another.)  The caller synchronises.
+template <typename T>
+__device__ __forceinline__ void copy_table(T& dst, const T& src) {
+    static_assert(sizeof(T) % 16 == 0, "whole 16-byte pieces");
+    for (unsigned i = threadIdx.x; i < sizeof(T) / 16; i += blockDim.x) reinterpret_cast<uint4*>(&dst)[i] = __ldg(reinterpret_cast<const uint4*>(&src) + i);
 }
+
+// Ordering between the kernels of one call.  They are launched so that a kernel's CTAs may be set up while the kernel
+// ahead of it drains; dependency_wait() returns once that one has finished and its writes are visible, and nothing but the
+// tables above is read before it.  dependents_may_launch() lets the next kernel's CTAs in as soon as all CTAs of this one run.
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // Nearest-code search, ties to the lower code: the number of midpoints strictly below x.  Same result
 // as the reference's q_mapping / bsearch including the end clamps (optim/cuda_adamw_kernels.cu:167-194,

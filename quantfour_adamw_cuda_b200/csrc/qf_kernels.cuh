@@ -123,7 +123,7 @@ struct Sched {
     int32_t rows;
     int32_t n_hypers;
 };
-// The sets of the current row, widened, into shared memory; the caller's next __syncthreads() publishes them.
+// The sets of the current row, widened, into shared memory; the caller synchronises.
 __device__ __forceinline__ void load_sched(HyperDev* sh, const Sched& sc) {
     if (threadIdx.x < sc.n_hypers) {
         const int32_t r = min(max(sc.counters[0], 0), sc.rows - 1);
@@ -176,41 +176,55 @@ constexpr Lut make_lut() {
     }
     return t;
 }
-__device__ const Lut g_mlut = make_lut();
-
 // Shared memory of a CTA: the 16-entry tables (exact path), the first-moment search table, and two
 // byte-indexed pair tables for the fast dequantize: a byte of packed codes (two elements) fetches the two
 // map values of either moment with one 64-bit load.
-// What the first pass needs of it.
-struct SmemPre {
-    Tables t;
-    float2 qv2[256];
+struct PairTable {
+    alignas(16) float2 v[256];   // (map[b & 15], map[b >> 4])
 };
-__device__ __forceinline__ void load_smem(SmemPre& s) {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) s.qv2[i] = make_float2(c_qv[i & 15], c_qv[i >> 4]);
-    load_tables(s.t);  // ends with __syncthreads()
-}
 struct Smem {
-    Tables t;
+    alignas(16) Tables t;
     alignas(16) uint8_t mlut[2048];
-    float2 qm2[256];   // (qm[b & 15], qm[b >> 4])
-    float2 qv2[256];   // (qv[b & 15], qv[b >> 4])
+    PairTable qm2, qv2;
 };
-
-__device__ __forceinline__ void load_smem(Smem& s) {
-    for (int i = threadIdx.x; i < 512; i += blockDim.x)
-        reinterpret_cast<uint32_t*>(s.mlut)[i] = reinterpret_cast<const uint32_t*>(g_mlut.base)[i];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        s.qm2[i] = make_float2(c_qm[i & 15], c_qm[i >> 4]);
-        s.qv2[i] = make_float2(c_qv[i & 15], c_qv[i >> 4]);
+struct SmemPre {   // what the first pass needs of it
+    alignas(16) Tables t;
+    PairTable qv2;
+};
+constexpr Smem make_smem() {
+    Smem s{};
+    const Lut lut = make_lut();
+    for (int i = 0; i < 16; ++i) {
+        s.t.qm[i] = kQm[i];
+        s.t.mm[i] = kMm[i];
+        s.t.qv[i] = kQv[i];
+        s.t.mv[i] = kMv[i];
     }
-    load_tables(s.t);  // ends with __syncthreads()
+    for (int i = 0; i < 2048; ++i) s.mlut[i] = lut.base[i];
+    for (int i = 0; i < 256; ++i) {
+        s.qm2.v[i].x = kQm[i & 15];
+        s.qm2.v[i].y = kQm[i >> 4];
+        s.qv2.v[i].x = kQv[i & 15];
+        s.qv2.v[i].y = kQv[i >> 4];
+    }
+    return s;
+}
+__device__ const Smem g_smem = make_smem();
+
+__device__ __forceinline__ void load_smem(SmemPre& s) {
+    copy_table(s.t, g_smem.t);
+    copy_table(s.qv2, g_smem.qv2);
+    __syncthreads();
+}
+__device__ __forceinline__ void load_smem(Smem& s) {
+    copy_table(s, g_smem);
+    __syncthreads();
 }
 
 // Entry of a pair table for byte j (elements 2j, 2j+1) of a word of eight codes.
-__device__ __forceinline__ f2 pair_lookup(const float2* tab, uint32_t w, int j) {
+__device__ __forceinline__ f2 pair_lookup(const PairTable& tab, uint32_t w, int j) {
     const uint32_t off = j == 0 ? (w << 3) & 0x7f8u : (w >> (8 * j - 3)) & 0x7f8u;
-    return *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(tab) + off);
+    return *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(tab.v) + off);
 }
 
 // `mid`: the 15 midpoints in ascending order followed by +inf (Tables::mm).
@@ -277,7 +291,7 @@ __device__ __forceinline__ int ceil_s32(float y) {
 }
 // The pair table entry of byte j of a word of eight codes, and the first-moment code of x, both with the plain
 // index (the scaling by the entry size folds into the shared-memory address).
-__device__ __forceinline__ f2 pair_entry(const float2* tab, uint32_t w, int j) { return tab[byte_of(w, j)]; }
+__device__ __forceinline__ f2 pair_entry(const PairTable& tab, uint32_t w, int j) { return tab.v[byte_of(w, j)]; }
 
 // A scale the fast division sequences may be used with.
 __device__ __forceinline__ bool scale_safe(float s) { return s == 0.0f || (s >= 0x1p-90f && s <= 0x1p100f); }
@@ -363,12 +377,6 @@ __device__ __forceinline__ float code_plus_2p23(uint32_t w, int k) {
 }
 constexpr float kMagic = -8388607.0f;
 
-// Exact quantization of four pairs, out of line: the rarely taken branch of the fast rows.
-__device__ __noinline__ uint32_t quantize8_pairs_exact(f2 a, f2 b, f2 c, f2 d, float scale, const float* mid) {
-    const float x[8] = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
-    return quantize8(x, scale, mid, 8);
-}
-
 // First-moment codes of a lane's 8 values against a block scale that the division sequences may be used with.
 __device__ __forceinline__ uint32_t quantize_m8_safe(const f2 (&m)[4], float scale, const Smem& s) {
     const Recip rc = make_recip(scale);  // 0 for an all-zero block: every quotient is 0
@@ -381,12 +389,6 @@ __device__ __forceinline__ uint32_t quantize_m8_safe(const f2 (&m)[4], float sca
         w += search_m_lut(q.y, s.mlut, s.t.mm) << (8 * j + 4);
     }
     return w;
-}
-
-// The same for any scale: fast division when it allows.
-__device__ __forceinline__ uint32_t quantize_m8(const f2 (&m)[4], float scale, const Smem& s) {
-    if (!scale_safe(scale)) return quantize8_pairs_exact(m[0], m[1], m[2], m[3], scale, s.t.mm);
-    return quantize_m8_safe(m, scale, s);
 }
 
 // Max of |x| over the 128-element block a lane's 8 values belong to (16 lanes), by redux instructions on the
@@ -1044,73 +1046,87 @@ __device__ __noinline__ void main_flat_run_exact(const DevTensor* tp, int64_t wb
     }
 }
 
-// One full, vector-aligned run of 256 elements with the packed arithmetic (block-128 and fp32-state kinds).
-template <typename T, int KIND>
-__device__ __forceinline__ void main_flat_run_fast(const DevTensor& t, int64_t wbase, const Hyper2& h2, const Smem& s,
-                                                   uint32_t* status, const PushPack* push) {
-    const int lane = threadIdx.x & 31;
-    const int64_t e = wbase + lane * 8;
-    float p[8], g[8];
+// One full, vector-aligned run of 256 elements with the packed arithmetic (fp32-state kind).
+template <typename T>
+__device__ __forceinline__ void main_flat_run_fp32(const DevTensor& t, int64_t wbase, const Hyper2& h2, const PushPack* push) {
+    const int64_t e = wbase + (threadIdx.x & 31) * 8;
+    float p[8], g[8], m[8], v[8];
     Elem<T>::load8(t.p, e, p);
     Elem<T>::load8(t.g, e, g);
-    if (KIND == QF_KIND_FP32) {
-        float m[8], v[8];
-        Elem<float>::load8(t.m, e, m);
-        Elem<float>::load8(t.v, e, v);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            f2 pp = mk2(p[2 * j], p[2 * j + 1]), mm = mk2(m[2 * j], m[2 * j + 1]), vv = mk2(v[2 * j], v[2 * j + 1]);
-            adamw_pair(pp, mk2(g[2 * j], g[2 * j + 1]), mm, vv, h2);
-            p[2 * j] = pp.x; p[2 * j + 1] = pp.y;
-            m[2 * j] = mm.x; m[2 * j + 1] = mm.y;
-            v[2 * j] = vv.x; v[2 * j + 1] = vv.y;
-        }
-        Elem<T>::store8(t.p, e, p);
-        if (push) push_store8<T>(t.p, e, p, push);
-        Elem<float>::store8(t.m, e, m);
-        Elem<float>::store8(t.v, e, v);
-        return;
-    }
-    uint8_t* mc = reinterpret_cast<uint8_t*>(t.m);
-    uint8_t* vc = reinterpret_cast<uint8_t*>(t.v);
-    const uint32_t wm = *reinterpret_cast<const uint32_t*>(mc + (e >> 1));
-    const uint32_t wv = *reinterpret_cast<const uint32_t*>(vc + (e >> 1));
-    const f2 ms_old = bc2(__ldg(t.ms + (e >> 7)));
-    const float vs_old = __ldg(t.vs + (e >> 7));
-    const f2 vs2 = bc2(vs_old);
-    f2 m[4], v[4];
+    Elem<float>::load8(t.m, e, m);
+    Elem<float>::load8(t.v, e, v);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        f2 pp = mk2(p[2 * j], p[2 * j + 1]);
-        m[j] = mul2(pair_lookup(s.qm2, wm, j), ms_old);
-        v[j] = mul2(pair_lookup(s.qv2, wv, j), vs2);
-        adamw_pair(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v[j], h2);
-        p[2 * j] = pp.x;
-        p[2 * j + 1] = pp.y;
+        f2 pp = mk2(p[2 * j], p[2 * j + 1]), mm = mk2(m[2 * j], m[2 * j + 1]), vv = mk2(v[2 * j], v[2 * j + 1]);
+        adamw_pair(pp, mk2(g[2 * j], g[2 * j + 1]), mm, vv, h2);
+        p[2 * j] = pp.x; p[2 * j + 1] = pp.y;
+        m[2 * j] = mm.x; m[2 * j + 1] = mm.y;
+        v[2 * j] = vv.x; v[2 * j + 1] = vv.y;
     }
     Elem<T>::store8(t.p, e, p);
     if (push) push_store8<T>(t.p, e, p, push);
+    Elem<float>::store8(t.m, e, m);
+    Elem<float>::store8(t.v, e, v);
+}
+
+// A lane's inputs of one full run of a block-128 tensor, as loaded.
+template <typename T>
+struct BlockRun {
+    Raw8<T> p, g;
+    uint32_t wm, wv;
+    float ms, vs;
+    __device__ __forceinline__ void load(const DevTensor& t, int64_t e) {
+        p.load(t.p, e);
+        g.load(t.g, e);
+        wm = *reinterpret_cast<const uint32_t*>(t.m + (e >> 1));
+        wv = *reinterpret_cast<const uint32_t*>(t.v + (e >> 1));
+        ms = t.ms[e >> 7];
+        vs = t.vs[e >> 7];
+    }
+};
+
+// One full run of a block-128 tensor with the packed arithmetic.  False: some value of the run leaves the ranges of the
+// sequences (a second moment below 2^-96, a new scale outside the range of the division; a NaN or infinity does the
+// latter); nothing of the run has been stored.
+template <typename T>
+__device__ __forceinline__ bool main_flat_run_block(const DevTensor& t, int64_t e, const BlockRun<T>& in, const Hyper2& h2, const Smem& s,
+                                                    const PushPack* push) {
+    float p[8], g[8];
+    in.p.widen(p);
+    in.g.widen(g);
+    const f2 ms_old = bc2(in.ms), vs_old = bc2(in.vs);
+    f2 m[4], v[4];
+    float low = __builtin_huge_valf();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        f2 pp = mk2(p[2 * j], p[2 * j + 1]);
+        m[j] = mul2(pair_entry(s.qm2, in.wm, j), ms_old);
+        v[j] = mul2(pair_entry(s.qv2, in.wv, j), vs_old);
+        adamw_pair<true>(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v[j], h2);
+        low = fminf(low, fminf(v[j].x, v[j].y));
+        p[2 * j] = pp.x;
+        p[2 * j + 1] = pp.y;
+    }
     const float ms_new = absmax_pairs_to_block_nan(m);   // no first pass vouches for these values: a NaN must survive
     const float vs_new = absmax_pairs_to_block_nan(v);
-    *reinterpret_cast<uint32_t*>(mc + (e >> 1)) = quantize_m8(m, ms_new, s);
-    uint32_t wq = 0;
-    if (scale_safe(vs_new)) {
-        const f2 r2 = bc2(vs_new == 0.0f ? 0.0f : __frcp_rn(vs_new)), ns2 = bc2(-vs_new);
+    if (!__all_sync(kFull, low >= 0x1p-96f && scale_safe(ms_new) && scale_safe(vs_new))) return false;
+    Elem<T>::store8(t.p, e, p);
+    if (push) push_store8<T>(t.p, e, p, push);
+    *reinterpret_cast<uint32_t*>(t.m + (e >> 1)) = quantize_m8_safe(m, ms_new, s);
+    const f2 r2 = bc2(__frcp_rn(vs_new)), ns2 = bc2(-vs_new);
+    int c[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const f2 y = fma2(div2_prepared(v[j], r2, ns2), bc2(16.0f), bc2(-1.5f));
-            wq += code_from_y<false>(y.x) << (8 * j);
-            wq += code_from_y<false>(y.y) << (8 * j + 4);
-        }
-    } else {
-        wq = quantize8_pairs_exact(v[0], v[1], v[2], v[3], vs_new, s.t.mv);
+    for (int j = 0; j < 4; ++j) {
+        const f2 y = fma2(div2_prepared(v[j], r2, ns2), bc2(16.0f), bc2(-1.5f));
+        c[2 * j] = ceil_s32(y.x);   // at most 15: the scale is the maximum of these values
+        c[2 * j + 1] = ceil_s32(y.y);
     }
-    *reinterpret_cast<uint32_t*>(vc + (e >> 1)) = wq;
-    if ((lane & 15) == 0) {
+    *reinterpret_cast<uint32_t*>(t.v + (e >> 1)) = pack_u4(c[1], c[0], pack_u4(c[3], c[2], pack_u4(c[5], c[4], pack_u4(c[7], c[6], 0u))));
+    if ((threadIdx.x & 15) == 0) {
         t.ms[e >> 7] = ms_new;
         t.vs[e >> 7] = vs_new;
-        if (nonfinite(ms_new) || nonfinite(vs_new)) atomicOr(status, QF_STATUS_NONFINITE);
     }
+    return true;
 }
 
 template <typename T, int KIND>
@@ -1118,13 +1134,12 @@ __device__ __forceinline__ void main_flat(const DevTensor* tp, int64_t li, const
                                           uint32_t* status, const PushPack* push) {
     const DevTensor t = *tp;
     const bool vec = t.flags & kFlagVec;
+    const int lane = threadIdx.x & 31;
     const int64_t start = li * (static_cast<int64_t>(kPanelCols) * t.flat_runs);
     const Hyper2 h2 = widen(hd);
-    for (int it = 0; it < t.flat_runs; ++it) {
-        const int64_t wbase = start + static_cast<int64_t>(it) * kPanelCols;
-        if (wbase >= t.numel) break;  // warp-uniform
-        if (KIND != QF_KIND_RANK1 && hd.gs != 1.0f) {  // no first pass for these kinds: the gradient is scaled here
-            const int64_t e = wbase + (threadIdx.x & 31) * 8;
+    if (KIND != QF_KIND_RANK1 && hd.gs != 1.0f) {  // no first pass for these kinds: the gradient is scaled here
+        for (int it = 0; it < t.flat_runs; ++it) {
+            const int64_t e = start + static_cast<int64_t>(it) * kPanelCols + lane * 8;
             const int nv = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(8), t.numel - e)));
             float g[8];
             load8_masked<T>(t.g, e, nv, vec, g);
@@ -1132,10 +1147,28 @@ __device__ __forceinline__ void main_flat(const DevTensor* tp, int64_t li, const
             for (int k = 0; k < 8; ++k) g[k] = round_as<T>(__fmul_rn(g[k], hd.gs));
             store8_masked<T>(const_cast<char*>(t.g), e, nv, vec, g);
         }
-        if (KIND != QF_KIND_RANK1 && hd.fast && vec && wbase + kPanelCols <= t.numel)
-            main_flat_run_fast<T, KIND>(t, wbase, h2, s, status, push);
-        else
-            main_flat_run_exact<T, KIND>(tp, wbase, hd, s, status, push);
+    }
+    // whole runs the packed arithmetic may take, then what is left
+    const int64_t whole = KIND != QF_KIND_RANK1 && hd.fast && vec ? max((t.numel - start) / kPanelCols, static_cast<int64_t>(0)) : 0;
+    const int fast = static_cast<int>(min(whole, static_cast<int64_t>(t.flat_runs)));
+    int it = 0;
+    if (KIND == QF_KIND_FP32) {
+        for (; it < fast; ++it) main_flat_run_fp32<T>(t, start + static_cast<int64_t>(it) * kPanelCols, h2, push);
+    } else if (KIND == QF_KIND_BLOCK && fast > 0) {
+        // the next run's inputs are requested before this run is worked on
+        int64_t e = start + lane * 8;
+        BlockRun<T> next;
+        next.load(t, e);
+        for (; it < fast; ++it, e += kPanelCols) {
+            const BlockRun<T> now = next;
+            if (it + 1 < fast) next.load(t, e + kPanelCols);
+            if (!main_flat_run_block<T>(t, e, now, h2, s, push)) main_flat_run_exact<T, KIND>(tp, e - lane * 8, hd, s, status, push);
+        }
+    }
+    for (; it < t.flat_runs; ++it) {
+        const int64_t wbase = start + static_cast<int64_t>(it) * kPanelCols;
+        if (wbase >= t.numel) break;  // warp-uniform
+        main_flat_run_exact<T, KIND>(tp, wbase, hd, s, status, push);
     }
 }
 
@@ -1403,6 +1436,8 @@ __device__ __forceinline__ void roll_item(const DevTensor* __restrict__ tensors,
 }
 __global__ void __launch_bounds__(kThreads)
 rank1_roll_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict__ base, int n, int mode) {
+    dependents_may_launch();
+    dependency_wait();
     roll_item(tensors, base, n, blockIdx.x, mode);
 }
 
@@ -1424,8 +1459,13 @@ step_pre_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict
                 const __grid_constant__ HyperPack hp, int ring_bytes, uint32_t* status, const __grid_constant__ Sched sc) {
     __shared__ SmemPre s;
     __shared__ HyperDev sched_h[SCHED ? QF_MAX_HYPERS : 1];
-    if (SCHED) load_sched(sched_h, sc);
+    dependents_may_launch();
     load_smem(s);
+    dependency_wait();
+    if (SCHED) {
+        load_sched(sched_h, sc);
+        __syncthreads();
+    }
     extern __shared__ __align__(16) char staging[];  // panel kernel: one ring of rows per warp
     char* stage = staging + (threadIdx.x >> 5) * ring_bytes;
     const int64_t total = base[n], per_cta = MAP == kMapFlat ? kWarpsPerCta : 1, stride = gridDim.x * per_cta;
@@ -1490,8 +1530,13 @@ step_main_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restric
     const PushPack* push = PUSH ? &pp : nullptr;
     __shared__ Smem s;
     __shared__ HyperDev sched_h[SCHED ? QF_MAX_HYPERS : 1];
-    if (SCHED) load_sched(sched_h, sc);
+    dependents_may_launch();
     load_smem(s);
+    dependency_wait();
+    if (SCHED) {
+        load_sched(sched_h, sc);
+        __syncthreads();
+    }
     extern __shared__ __align__(16) char staging[];  // panel kernel: per warp a ring of rows plus the column block
     char* stage = staging + (threadIdx.x >> 5) * (ring_bytes + kColBytes + kRowBufBytes);
     const int64_t total = base[n], per_cta = MAP == kMapStrip ? 1 : kWarpsPerCta, stride = gridDim.x * per_cta;
@@ -1533,7 +1578,9 @@ __device__ uint32_t g_unread_status;
 __global__ void __launch_bounds__(kThreads)
 single_tensor_kernel(const __grid_constant__ DevTensor t, const __grid_constant__ HyperDev h) {
     __shared__ Smem s;
+    dependents_may_launch();
     load_smem(s);
+    dependency_wait();
     const int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
     if (item * (static_cast<int64_t>(kPanelCols) * t.flat_runs) >= t.numel) return;
     if (t.dtype == QF_BF16)
@@ -1687,10 +1734,11 @@ __global__ void __launch_bounds__(kThreads)
 dequantize_block_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ scales, int64_t numel, int map,
                         float* __restrict__ out, int vec) {
     __shared__ Tables s;
-    __shared__ float2 pair[256];   // (value of the low nibble, value of the high nibble) of a byte of codes
-    for (int i = threadIdx.x; i < 256; i += blockDim.x)
-        pair[i] = map ? make_float2(c_qv[i & 15], c_qv[i >> 4]) : make_float2(c_qm[i & 15], c_qm[i >> 4]);
-    load_tables(s);  // ends with __syncthreads()
+    __shared__ PairTable table;
+    copy_table(s, g_smem.t);
+    copy_table(table, map ? g_smem.qv2 : g_smem.qm2);
+    __syncthreads();
+    const float2* pair = table.v;
     const float* q = map ? s.qv : s.qm;
     const int lane = threadIdx.x & 31;
     const int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
@@ -1740,9 +1788,10 @@ dequantize_block_kernel(const uint8_t* __restrict__ codes, const float* __restri
 __global__ void __launch_bounds__(kThreads)
 rank1_dequant_panel_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ row_max, const float* __restrict__ col_max,
                            int rows, int cols, float* __restrict__ out) {
-    __shared__ float2 pair[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) pair[i] = make_float2(c_qv[i & 15], c_qv[i >> 4]);
+    __shared__ PairTable table;
+    copy_table(table, g_smem.qv2);
     __syncthreads();
+    const float2* pair = table.v;
     const int lane = threadIdx.x & 31;
     const int panels = cols / kPanelCols;
     const int64_t total = static_cast<int64_t>((rows + kRowsPerItem - 1) / kRowsPerItem) * panels;
@@ -1908,7 +1957,8 @@ __global__ void __launch_bounds__(kThreads)
 rank1_codec_kernel(const float* __restrict__ in, uint8_t* __restrict__ codes, const float* __restrict__ row_max,
                    const float* __restrict__ col_max, int rows, int cols, float* __restrict__ out, int vec) {
     __shared__ Tables s;
-    load_tables(s);
+    copy_table(s, g_smem.t);
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     const int64_t numel = static_cast<int64_t>(rows) * cols;
     const int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
