@@ -1,6 +1,7 @@
 // Host side of libquantfour_b200.so: argument validation, the device descriptor table and the
 // launches.  The exported functions are declared and documented in include/quantfour_b200.h.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstddef>
@@ -135,6 +136,11 @@ int flat_runs_for(int64_t runs) {
     return item_length(runs, qf::kRowsPerItem, qf::kMinRowsPerItem, 1, 1, qf::kMainMinCtas * qf::kWarpsPerCta);
 }
 int strip_runs_for(int64_t runs) { return item_length(ceil_div(runs, qf::kWarpsPerCta), qf::kStripRuns, 1, 1, 1, qf::kMainMinCtas); }
+// The stand-alone quantize / dequantize kernels, five CTAs per SM by their registers: runs (or rows of a panel) per warp,
+// runs of a strip.
+constexpr int kCodecCtas = 5;
+int codec_runs_for(int64_t runs, int step) { return item_length(runs, qf::kRowsPerItem, step, step, 1, kCodecCtas * qf::kWarpsPerCta); }
+int codec_strip_runs_for(int64_t numel) { return item_length(ceil_div(numel, qf::strip_entries(1)), qf::kStripRuns, 1, 1, 1, kCodecCtas); }
 int64_t runs_of(int64_t numel) { return ceil_div(numel, qf::kPanelCols); }
 
 // The strip mapping takes a rank-1 tensor that is not whole panels if its buffers are vector-aligned and a lane's eight
@@ -318,10 +324,24 @@ unsigned persistent_grid(int64_t items, int per_sm, int waves = kGridWaves) {
     return static_cast<unsigned>(ctas < cap ? ctas : cap);
 }
 
-// A kernel of a step, launched so that it may be set up while the kernel ahead of it on the stream drains (every such
+// Room for `dyn_max` bytes of dynamic shared memory, asked for once per kernel and device.
+template <auto Kernel>
+int prepare_kernel(int dyn_max) {
+    static std::atomic<uint64_t> done{0};   // a bit per device
+    if (dyn_max == 0) return QF_OK;
+    int dev = 0;
+    QF_CUDA(cudaGetDevice(&dev));
+    if (dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1)) return QF_OK;
+    QF_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_max));
+    if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
+    return QF_OK;
+}
+
+// Launches a kernel of a step so that it may be set up while the kernel ahead of it on the stream drains (every such
 // kernel waits for that one's end before it touches memory: dependency_wait in qf_device.cuh).
-template <typename... Params, typename... Args>
-cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, size_t smem, cudaStream_t stream, Args... args) {
+template <auto Kernel, typename... Params, typename... Args>
+int launch_as(void (*)(Params...), unsigned grid, int smem, int smem_max, cudaStream_t stream, Args... args) {
+    if (int rc = prepare_kernel<Kernel>(smem_max)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(qf::kThreads);
@@ -332,12 +352,16 @@ cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, size_t smem
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    QF_CUDA(cudaLaunchKernelEx(&cfg, Kernel, static_cast<Params>(args)...));
+    return QF_OK;
+}
+template <auto Kernel, typename... Args>
+int launch_chained(unsigned grid, int smem, int smem_max, cudaStream_t stream, Args... args) {
+    return launch_as<Kernel>(Kernel, grid, smem, smem_max, stream, args...);
 }
 
 int roll(const Plan& pl, int mode, cudaStream_t stream) {
-    QF_CUDA(launch_chained(qf::rank1_roll_kernel, static_cast<unsigned>(pl.items[kRoll]), 0, stream, pl.d_tensors, pl.d_base[kRoll], pl.n, mode));
-    return QF_OK;
+    return launch_chained<qf::rank1_roll_kernel>(static_cast<unsigned>(pl.items[kRoll]), 0, 0, stream, pl.d_tensors, pl.d_base[kRoll], pl.n, mode);
 }
 
 qf::Sched no_sched() {
@@ -353,23 +377,22 @@ unsigned cta_grid(int64_t items, int per_sm) {   // one item per CTA and turn
 template <bool SCALE, bool SCHED>
 int launch_pre_panel(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
     const int dyn = qf::pre_dyn_smem(pl.any_f32_panel);
-    QF_CUDA(cudaFuncSetAttribute(qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED>, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::pre_dyn_smem(true)));
-    QF_CUDA(launch_chained(qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED>, cta_grid(pl.items[kPrePanel], qf::kPreMinCtas), dyn, stream,
-                           pl.d_tensors, pl.d_base[kPrePanel], pl.n, hp, dyn / qf::kWarpsPerCta, pl.d_status, sc));
-    return QF_OK;
+    return launch_chained<qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED>>(
+        cta_grid(pl.items[kPrePanel], qf::kPreMinCtas), dyn, qf::pre_dyn_smem(true), stream, pl.d_tensors, pl.d_base[kPrePanel], pl.n, hp,
+        dyn / qf::kWarpsPerCta, pl.d_status, sc);
 }
 
 // First pass over the strips and over the flat items; the kernels see by themselves whether a gradient scale is set.
 template <bool SCHED>
 int launch_pre_others(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
-    if (pl.items[kStrip]) {
-        auto* kernel = qf::step_pre_kernel<qf::kMapStrip, false, SCHED>;
-        QF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::strip_dyn_smem()));
-        QF_CUDA(launch_chained(kernel, cta_grid(pl.items[kStrip], qf::kPreMinCtas), qf::strip_dyn_smem(), stream, pl.d_tensors, pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, sc));
-    }
+    if (pl.items[kStrip])
+        if (int rc = launch_chained<qf::step_pre_kernel<qf::kMapStrip, false, SCHED>>(
+                cta_grid(pl.items[kStrip], qf::kPreMinCtas), qf::strip_dyn_smem(), qf::strip_dyn_smem(), stream, pl.d_tensors,
+                pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, sc))
+            return rc;
     if (pl.items[kPreFlat])
-        QF_CUDA(launch_chained(qf::step_pre_kernel<qf::kMapFlat, false, SCHED>, persistent_grid(pl.items[kPreFlat], qf::kPreMinCtas), 0, stream,
-                               pl.d_tensors, pl.d_base[kPreFlat], pl.n, hp, 0, pl.d_status, sc));
+        return launch_chained<qf::step_pre_kernel<qf::kMapFlat, false, SCHED>>(
+            persistent_grid(pl.items[kPreFlat], qf::kPreMinCtas), 0, 0, stream, pl.d_tensors, pl.d_base[kPreFlat], pl.n, hp, 0, pl.d_status, sc);
     return QF_OK;
 }
 
@@ -400,11 +423,9 @@ template <bool PUSH, bool BC1, bool SCHED, bool RELAXED, int DT>
 int launch_main_panel_dt(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, cudaStream_t stream) {
     const int dyn = qf::main_dyn_smem(pl.any_f32_panel);
     const int ring = qf::kStages * (pl.any_f32_panel ? qf::kRowBytesF32 : qf::kRowBytesBf16);
-    QF_CUDA(cudaFuncSetAttribute(qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 qf::main_dyn_smem(true)));
-    QF_CUDA(launch_chained(qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT>, persistent_grid(pl.items[kMainPanel], qf::kMainMinCtas), dyn, stream,
-                           pl.d_tensors, pl.d_base[kMainPanel], pl.n, hp, ring, pl.d_status, pp, sc, pl.d_base[kRoll], static_cast<int>(pl.items[kRoll])));
-    return QF_OK;
+    return launch_chained<qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT>>(
+        persistent_grid(pl.items[kMainPanel], qf::kMainMinCtas), dyn, qf::main_dyn_smem(true), stream, pl.d_tensors, pl.d_base[kMainPanel],
+        pl.n, hp, ring, pl.d_status, pp, sc, pl.d_base[kRoll], static_cast<int>(pl.items[kRoll]));
 }
 // A launch whose panel tensors are all of one dtype takes the kernel that carries that dtype's loop only (the plain
 // step, the common case; the rarer variants keep the two-dtype kernel): 1.4 % faster, measured.
@@ -423,14 +444,16 @@ template <bool PUSH, bool SCHED>
 int launch_main_others(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, cudaStream_t stream) {
     int rolls = pl.items[kMainPanel] ? 0 : static_cast<int>(pl.items[kRoll]);
     if (pl.items[kStrip]) {
-        auto* kernel = qf::step_main_kernel<qf::kMapStrip, PUSH, false, SCHED>;
-        QF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, qf::strip_dyn_smem()));
-        QF_CUDA(launch_chained(kernel, cta_grid(pl.items[kStrip], qf::kMainMinCtas), qf::strip_dyn_smem(), stream, pl.d_tensors, pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls));
+        if (int rc = launch_chained<qf::step_main_kernel<qf::kMapStrip, PUSH, false, SCHED>>(
+                cta_grid(pl.items[kStrip], qf::kMainMinCtas), qf::strip_dyn_smem(), qf::strip_dyn_smem(), stream, pl.d_tensors,
+                pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls))
+            return rc;
         rolls = 0;
     }
     if (pl.items[kMainFlat])
-        QF_CUDA(launch_chained(qf::step_main_kernel<qf::kMapFlat, PUSH, false, SCHED>, persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), 0, stream,
-                               pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls));
+        return launch_chained<qf::step_main_kernel<qf::kMapFlat, PUSH, false, SCHED>>(
+            persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), 0, 0, stream, pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status,
+            pp, sc, pl.d_base[kRoll], rolls);
     return QF_OK;
 }
 
@@ -504,10 +527,6 @@ int check_1d(const void* a, const void* b, int64_t numel, const char* what) {
     if (numel < 0) return fail(QF_ERR_BAD_ARG, "%s: negative numel", what);
     if (numel > 0 && (!a || !b)) return fail(QF_ERR_BAD_ARG, "%s: null pointer", what);
     return QF_OK;
-}
-
-unsigned flat_grid(int64_t numel) {
-    return static_cast<unsigned>((flat_items(numel) + qf::kWarpsPerCta - 1) / qf::kWarpsPerCta);
 }
 
 // Grid of single_tensor_kernel: one item per warp.
@@ -799,9 +818,7 @@ int qf_fused_4bit(void* p, const void* g, void* exp, void* sq, float* exp_scale,
     QfHyper h;
     qf_make_hyper(lr, beta1, beta2, eps, weight_decay, step, &h);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    QF_CUDA(launch_chained(qf::single_tensor_kernel, single_grid(t), 0, st, t, widen_hyper(h)));
-    QF_CUDA(cudaGetLastError());
-    return QF_OK;
+    return launch_chained<qf::single_tensor_kernel>(single_grid(t), 0, 0, st, t, widen_hyper(h));
 }
 
 int qf_fused_single_tensor(void* p, const void* g, float* exp_avg, float* exp_avg_sq, int64_t numel, int dtype,
@@ -829,9 +846,7 @@ int qf_fused_single_tensor(void* p, const void* g, float* exp_avg, float* exp_av
     QfHyper h;
     qf_make_hyper(lr, beta1, beta2, eps, weight_decay, step, &h);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    QF_CUDA(launch_chained(qf::single_tensor_kernel, single_grid(t), 0, st, t, widen_hyper(h)));
-    QF_CUDA(cudaGetLastError());
-    return QF_OK;
+    return launch_chained<qf::single_tensor_kernel>(single_grid(t), 0, 0, st, t, widen_hyper(h));
 }
 
 int qf_quantize_block(const float* x, int64_t numel, int map, uint8_t* codes, float* scales, int device, void* stream) {
@@ -843,11 +858,12 @@ int qf_quantize_block(const float* x, int64_t numel, int map, uint8_t* codes, fl
     if (!aligned(x, 4) || !aligned(scales, 4)) return fail(QF_ERR_BAD_ARG, "qf_quantize_block: x / scales not 4-byte aligned");
     QF_CUDA(cudaSetDevice(device));
     const int vec = aligned(x, 16) && aligned(codes, 4);
-    const unsigned grid = persistent_grid(flat_items(numel), 8, 2);
+    const int runs = codec_runs_for(runs_of(numel), 1);
+    const unsigned grid = persistent_grid(ceil_div(runs_of(numel), runs), kCodecCtas);
     if (map)
-        qf::quantize_block_kernel<1><<<grid, qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(x, numel, codes, scales, vec);
+        qf::quantize_block_kernel<1><<<grid, qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(x, numel, codes, scales, vec, runs);
     else
-        qf::quantize_block_kernel<0><<<grid, qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(x, numel, codes, scales, vec);
+        qf::quantize_block_kernel<0><<<grid, qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(x, numel, codes, scales, vec, runs);
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -862,8 +878,10 @@ int qf_dequantize_block(const uint8_t* codes, const float* scales, int64_t numel
     if (!aligned(out, 4) || !aligned(scales, 4)) return fail(QF_ERR_BAD_ARG, "qf_dequantize_block: out / scales not 4-byte aligned");
     QF_CUDA(cudaSetDevice(device));
     const int vec = aligned(out, 16) && aligned(codes, 4);
-    qf::dequantize_block_kernel<<<flat_grid(numel), qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(codes, scales, numel,
-                                                                                                        map, out, vec);
+    const int runs = codec_runs_for(runs_of(numel), 4);
+    unsigned grid;
+    if (int rc = grid_for(ceil_div(runs_of(numel), runs), &grid)) return rc;
+    qf::dequantize_block_kernel<<<grid, qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(codes, scales, numel, map, out, vec, runs);
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -882,18 +900,26 @@ int qf_quantize_rank1(const float* v, int64_t rows, int64_t cols, uint8_t* codes
     QF_CUDA(cudaMemsetAsync(row_max, 0, sizeof(float) * rows, st));
     QF_CUDA(cudaMemsetAsync(col_max, 0, sizeof(float) * cols, st));
     const int vec = aligned(v, 16) && aligned(codes, 4);
-    const int panel = vec && cols % qf::kPanelCols == 0;
-    const int64_t items = panel ? (rows + qf::kRowsPerItem - 1) / qf::kRowsPerItem * (cols / qf::kPanelCols) : flat_items(numel);
-    const int64_t max_items = panel ? (rows + qf::kPreRowsPerItem - 1) / qf::kPreRowsPerItem * (cols / qf::kPanelCols) : items;
-    unsigned grid;
-    if (int rc = grid_for(max_items, &grid)) return rc;
-    qf::rank1_max_kernel<<<grid, qf::kThreads, 0, st>>>(v, static_cast<int>(rows), static_cast<int>(cols), row_max, col_max, panel);
-    if (panel && aligned(col_max, 16))
-        qf::rank1_quant_panel_kernel<<<persistent_grid(items, 8), qf::kThreads, 0, st>>>(v, codes, row_max, col_max, static_cast<int>(rows),
-                                                                                      static_cast<int>(cols));
-    else
-        qf::rank1_codec_kernel<true><<<flat_grid(numel), qf::kThreads, 0, st>>>(v, codes, row_max, col_max, static_cast<int>(rows),
-                                                                               static_cast<int>(cols), nullptr, vec);
+    const int r = static_cast<int>(rows), c = static_cast<int>(cols);
+    if (vec && cols % qf::kPanelCols == 0 && aligned(col_max, 16)) {
+        const int64_t panels = cols / qf::kPanelCols;
+        const int max_rows = pre_rows_for(rows * panels), item_rows = codec_runs_for(rows * panels, 1);
+        const int64_t max_items = ceil_div(rows, static_cast<int64_t>(max_rows) * qf::kWarpsPerCta) * panels;
+        if (max_items > INT32_MAX) return fail(QF_ERR_BAD_ARG, "too many work items for one launch (%lld)", (long long)max_items);
+        qf::rank1_max_panel_kernel<<<static_cast<unsigned>(max_items), qf::kThreads, 0, st>>>(v, r, c, row_max, col_max, max_rows);
+        qf::rank1_quant_panel_kernel<<<persistent_grid(ceil_div(rows, item_rows) * panels, kCodecCtas), qf::kThreads, 0, st>>>(
+            v, codes, row_max, col_max, r, c, item_rows);
+    } else if (strip_fits(cols, vec)) {
+        const int runs = codec_strip_runs_for(numel);
+        const unsigned grid = static_cast<unsigned>(ceil_div(numel, qf::strip_entries(runs)));   // at most 2^62 / 2^13, and memory ends far below 2^43
+        qf::rank1_max_strip_kernel<<<grid, qf::kThreads, qf::strip_dyn_smem() / 2, st>>>(v, r, c, row_max, col_max, runs);
+        qf::rank1_codec_strip_kernel<true><<<grid, qf::kThreads, qf::strip_dyn_smem() / 2, st>>>(v, codes, row_max, col_max, r, c, nullptr, runs);
+    } else {
+        unsigned grid;
+        if (int rc = grid_for(flat_items(numel), &grid)) return rc;
+        qf::rank1_max_kernel<<<grid, qf::kThreads, 0, st>>>(v, r, c, row_max, col_max);
+        qf::rank1_codec_kernel<true><<<grid, qf::kThreads, 0, st>>>(v, codes, row_max, col_max, r, c, nullptr, vec);
+    }
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
@@ -909,13 +935,21 @@ int qf_dequantize_rank1(const uint8_t* codes, const float* row_max, const float*
         return fail(QF_ERR_BAD_ARG, "qf_dequantize_rank1: out / row_max / col_max not 4-byte aligned");
     QF_CUDA(cudaSetDevice(device));
     const int vec = aligned(out, 16) && aligned(codes, 4);
+    const int r = static_cast<int>(rows), c = static_cast<int>(cols);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (vec && cols % qf::kPanelCols == 0 && aligned(col_max, 16)) {
-        const int64_t items = (rows + qf::kRowsPerItem - 1) / qf::kRowsPerItem * (cols / qf::kPanelCols);
-        qf::rank1_dequant_panel_kernel<<<persistent_grid(items, 8), qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            codes, row_max, col_max, static_cast<int>(rows), static_cast<int>(cols), out);
+        const int64_t panels = cols / qf::kPanelCols;
+        const int item_rows = codec_runs_for(rows * panels, 1);
+        qf::rank1_dequant_panel_kernel<<<persistent_grid(ceil_div(rows, item_rows) * panels, kCodecCtas), qf::kThreads, 0, st>>>(
+            codes, row_max, col_max, r, c, out, item_rows);
+    } else if (strip_fits(cols, vec)) {
+        const int runs = codec_strip_runs_for(numel);
+        qf::rank1_codec_strip_kernel<false><<<static_cast<unsigned>(ceil_div(numel, qf::strip_entries(runs))), qf::kThreads,
+                                              qf::strip_dyn_smem() / 2, st>>>(nullptr, const_cast<uint8_t*>(codes), row_max, col_max, r, c, out, runs);
     } else {
-        qf::rank1_codec_kernel<false><<<flat_grid(numel), qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            nullptr, const_cast<uint8_t*>(codes), row_max, col_max, static_cast<int>(rows), static_cast<int>(cols), out, vec);
+        unsigned grid;
+        if (int rc = grid_for(flat_items(numel), &grid)) return rc;
+        qf::rank1_codec_kernel<false><<<grid, qf::kThreads, 0, st>>>(nullptr, const_cast<uint8_t*>(codes), row_max, col_max, r, c, out, vec);
     }
     QF_CUDA(cudaGetLastError());
     return QF_OK;

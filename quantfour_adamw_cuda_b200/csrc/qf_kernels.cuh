@@ -448,10 +448,14 @@ __device__ __forceinline__ void cp_async_wait() {
 // First pass over one item of a rank-1 panel: the work of a whole CTA, each warp taking `pre_rows` consecutive rows of the
 // panel's 256 columns.  This pass does little arithmetic per byte, so it needs many bytes in
 // flight to cover HBM latency: each lane stages its own 16-byte piece of g and its code word of the next
-// kPreStages - 1 rows into a per-warp ring with cp.async (a lane reads only what it copied, so no barrier), and the
+// stages - 1 rows into a per-warp ring with cp.async (a lane reads only what it copied, so no barrier), and the
 // old row maxima of the item are fetched up front, two per lane, and handed out by shuffle.
-constexpr int kPreStages = 8;
-constexpr int pre_dyn_smem(bool any_f32) { return kWarpsPerCta * kPreStages * 32 * ((any_f32 ? 32 : 16) + 4); }
+constexpr int kPreStages16 = 8;
+constexpr int kPreStages32 = 4;   // fp32 rows: 8 stages leave room for two CTAs per SM instead of three (4096 x 4096: 29.0 against 25.7 us)
+constexpr int pre_dyn_smem(bool any_f32) {
+    const int b16 = kPreStages16 * (16 + 4), b32 = kPreStages32 * (32 + 4);
+    return kWarpsPerCta * 32 * (any_f32 && b32 > b16 ? b32 : b16);
+}
 
 template <typename T, bool SCALE>
 __device__ __forceinline__ void pre_panel(const DevTensor& t, int64_t li, const HyperDev& hd, const SmemPre& s,
@@ -468,6 +472,7 @@ __device__ __forceinline__ void pre_panel(const DevTensor& t, int64_t li, const 
     const uint8_t* vc = reinterpret_cast<const uint8_t*>(t.v);
     constexpr int NV = sizeof(T) / 2;
     constexpr int kRowBytes = 32 * (NV * 16 + 4);
+    constexpr int kPreStages = NV == 1 ? kPreStages16 : kPreStages32;
     const uint32_t cols = static_cast<uint32_t>(t.cols);
     auto issue = [&](uint32_t e, int slot) {
         char* base = stage + slot * kRowBytes;
@@ -1649,19 +1654,19 @@ __global__ void sched_advance_kernel(int32_t* counters, int rows, int tail_repea
 // Stand-alone quantize / dequantize kernels (fp32 in / out)
 // =================================================================================================
 
-// Block-128 quantize: one warp item = kRowsPerItem runs of 256 elements.  MAP: 0 first-moment map (table search),
+// Block-128 quantize: one warp item = `runs` (at most kRowsPerItem) runs of 256 elements.  MAP: 0 first-moment map (table search),
 // 1 second-moment map (closed form).  Items that lie wholly inside a vector-aligned tensor take a loop without
 // masks; the last item and unaligned tensors take the general one.
 template <int MAP>
 __global__ void __launch_bounds__(kThreads)
 quantize_block_kernel(const float* __restrict__ x, int64_t numel, uint8_t* __restrict__ codes, float* __restrict__ scales,
-                      int vec) {
+                      int vec, int runs) {
     __shared__ Smem s;
     load_smem(s);
     const float* mid = MAP ? s.t.mv : s.t.mm;
     const int lane = threadIdx.x & 31;
     // warps stride over the items, so that a CTA fills its search table once for many items
-    const int64_t per_item = static_cast<int64_t>(kPanelCols) * kRowsPerItem;
+    const int64_t per_item = static_cast<int64_t>(kPanelCols) * runs;
     const int64_t total = (numel + per_item - 1) / per_item, stride = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
     for (int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5); item < total; item += stride) {
         const int64_t start = item * per_item;
@@ -1673,9 +1678,9 @@ quantize_block_kernel(const float* __restrict__ x, int64_t numel, uint8_t* __res
             uint16_t* c16 = reinterpret_cast<uint16_t*>(codes + (start >> 1)) + lane;
             float* sc_out = scales + (start >> 7);
             float4 na = src[0], nb = src[32];  // the next run's input is requested before this run is worked on
-            for (int it = 0; it < kRowsPerItem; ++it) {
+            for (int it = 0; it < runs; ++it) {
                 const f2 va[2] = {mk2(na.x, na.y), mk2(na.z, na.w)}, vb[2] = {mk2(nb.x, nb.y), mk2(nb.z, nb.w)};
-                const int nx = it + 1 < kRowsPerItem ? it + 1 : it;  // past the end: read the last run again
+                const int nx = it + 1 < runs ? it + 1 : it;  // past the end: read the last run again
                 na = src[nx * 64];
                 nb = src[nx * 64 + 32];
                 // bit patterns, so that a NaN survives the maximum
@@ -1711,7 +1716,7 @@ quantize_block_kernel(const float* __restrict__ x, int64_t numel, uint8_t* __res
             }
             continue;
         }
-        for (int it = 0; it < kRowsPerItem; ++it) {
+        for (int it = 0; it < runs; ++it) {
             const int64_t wbase = start + static_cast<int64_t>(it) * kPanelCols;
             if (wbase >= numel) break;
             const int64_t e = wbase + lane * 8;
@@ -1732,7 +1737,7 @@ quantize_block_kernel(const float* __restrict__ x, int64_t numel, uint8_t* __res
 // The codes of a lane's two quads are two 16-bit loads (64 contiguous bytes per warp each).
 __global__ void __launch_bounds__(kThreads)
 dequantize_block_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ scales, int64_t numel, int map,
-                        float* __restrict__ out, int vec) {
+                        float* __restrict__ out, int vec, int runs) {   // runs per item: a multiple of 4
     __shared__ Tables s;
     __shared__ PairTable table;
     copy_table(s, g_smem.t);
@@ -1742,13 +1747,13 @@ dequantize_block_kernel(const uint8_t* __restrict__ codes, const float* __restri
     const float* q = map ? s.qv : s.qm;
     const int lane = threadIdx.x & 31;
     const int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
-    const int64_t start = item * (kPanelCols * kRowsPerItem);
-    if (vec && start + kPanelCols * kRowsPerItem <= numel) {  // warp-uniform: a whole item inside an aligned tensor
+    const int64_t start = item * (static_cast<int64_t>(kPanelCols) * runs);
+    if (vec && start + static_cast<int64_t>(kPanelCols) * runs <= numel) {  // warp-uniform: a whole item inside an aligned tensor
         const uint16_t* c16 = reinterpret_cast<const uint16_t*>(codes + (start >> 1)) + lane;
         const float* sc = scales + (start >> 7);
         float4* dst = reinterpret_cast<float4*>(out + start) + lane;
         // the code halves and scales of four runs are requested together, then expanded and stored
-        for (int it0 = 0; it0 < kRowsPerItem; it0 += 4) {
+        for (int it0 = 0; it0 < runs; it0 += 4) {
             uint32_t wa[4], wb[4];
             float sa[4], sb[4];
 #pragma unroll
@@ -1769,7 +1774,7 @@ dequantize_block_kernel(const uint8_t* __restrict__ codes, const float* __restri
         }
         return;
     }
-    for (int it = 0; it < kRowsPerItem; ++it) {
+    for (int it = 0; it < runs; ++it) {
         const int64_t e = start + static_cast<int64_t>(it) * kPanelCols + lane * 8;
         if (e >= numel) break;
         const int nv = static_cast<int>(min(static_cast<int64_t>(8), numel - e));
@@ -1787,19 +1792,19 @@ dequantize_block_kernel(const uint8_t* __restrict__ codes, const float* __restri
 // the maxima of its 8 columns in registers; the next row's codes are requested before this row is worked on.
 __global__ void __launch_bounds__(kThreads)
 rank1_dequant_panel_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ row_max, const float* __restrict__ col_max,
-                           int rows, int cols, float* __restrict__ out) {
+                           int rows, int cols, float* __restrict__ out, int item_rows) {
     __shared__ PairTable table;
     copy_table(table, g_smem.qv2);
     __syncthreads();
     const float2* pair = table.v;
     const int lane = threadIdx.x & 31;
     const int panels = cols / kPanelCols;
-    const int64_t total = static_cast<int64_t>((rows + kRowsPerItem - 1) / kRowsPerItem) * panels;
+    const int64_t total = static_cast<int64_t>((rows + item_rows - 1) / item_rows) * panels;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
     for (int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5); item < total; item += stride) {
         const int band = static_cast<int>(item / panels);
         const int c0 = static_cast<int>(item - static_cast<int64_t>(band) * panels) * kPanelCols;   // first column of the panel
-        const int r0 = band * kRowsPerItem, r1 = min(r0 + kRowsPerItem, rows);
+        const int r0 = band * item_rows, r1 = min(r0 + item_rows, rows);
         const float4 ca = __ldg(reinterpret_cast<const float4*>(col_max + c0) + lane);
         const float4 cb = __ldg(reinterpret_cast<const float4*>(col_max + c0 + 128) + lane);
         const uint16_t* c16 = reinterpret_cast<const uint16_t*>(codes) + lane;
@@ -1825,67 +1830,241 @@ rank1_dequant_panel_kernel(const uint8_t* __restrict__ codes, const float* __res
     }
 }
 
-// Row / column maxima of |v| for an [R, C] fp32 matrix.  panel != 0: C is a multiple of 256 and the
-// buffers are vector-aligned; otherwise per-element atomics.
+// Row / column maxima of |v| for an [R, C] fp32 matrix whose columns are whole panels and whose buffers are vector-aligned.
+// An item is a CTA's: each warp takes `item_rows` rows of the panel, the warps' column maxima are combined before the
+// atomics (one red.max per column for eight times as many rows).
 __global__ void __launch_bounds__(kThreads)
-rank1_max_kernel(const float* __restrict__ v, int rows, int cols, float* __restrict__ row_max,
-                 float* __restrict__ col_max, int panel) {
-    const int lane = threadIdx.x & 31;
-    const int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
-    if (panel) {
-        const int panels = cols / kPanelCols;
-        const int band = static_cast<int>(item / panels);
-        const int r0 = band * kPreRowsPerItem;  // tall items: one column atomic per 64 rows
-        if (r0 >= rows) return;
-        const int r1 = min(r0 + kPreRowsPerItem, rows);
-        // lane L takes columns 4L .. 4L+3 and 128+4L .. 128+4L+3 of the panel: each of its two 128-bit loads is one of
-        // 32 consecutive 16-byte pieces, a load instruction of the warp reads 512 contiguous bytes
-        const int c0 = static_cast<int>(item - static_cast<int64_t>(band) * panels) * kPanelCols;
-        uint32_t cmax[8];
+rank1_max_panel_kernel(const float* __restrict__ v, int rows, int cols, float* __restrict__ row_max, float* __restrict__ col_max,
+                       int item_rows) {
+    __shared__ uint32_t warp_max[kWarpsPerCta][kPanelCols];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int panels = cols / kPanelCols;
+    const int band = static_cast<int>(blockIdx.x / panels);
+    const int r0 = min((band * kWarpsPerCta + warp) * item_rows, rows), r1 = min(r0 + item_rows, rows);
+    // lane L takes columns 4L .. 4L+3 and 128+4L .. 128+4L+3 of the panel: each of its two 128-bit loads is one of
+    // 32 consecutive 16-byte pieces, a load instruction of the warp reads 512 contiguous bytes
+    const int c0 = static_cast<int>(blockIdx.x - static_cast<unsigned>(band) * panels) * kPanelCols;
+    uint32_t cmax[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) cmax[k] = 0;
-        // four rows are requested together (4 KB per warp in flight): this pass does almost no arithmetic and
-        // lives on memory-level parallelism.  Past the last row the last row is read again, which changes no maximum.
-        for (int rb = r0; rb < r1; rb += 4) {
-            float x[4][8];
+    for (int k = 0; k < 8; ++k) cmax[k] = 0;
+    // four rows are requested together (4 KB per warp in flight): this pass does almost no arithmetic and
+    // lives on memory-level parallelism.  Past the last row the last row is read again, which changes no maximum.
+    for (int rb = r0; rb < r1; rb += 4) {
+        float x[4][8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4* src = reinterpret_cast<const float4*>(v + static_cast<int64_t>(min(rb + i, r1 - 1)) * cols + c0) + lane;
-                const float4 a = __ldg(src), b = __ldg(src + 32);
-                x[i][0] = a.x; x[i][1] = a.y; x[i][2] = a.z; x[i][3] = a.w;
-                x[i][4] = b.x; x[i][5] = b.y; x[i][6] = b.z; x[i][7] = b.w;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t rmax = 0;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const uint32_t b = absbits(x[i][k]);
-                    rmax = max(rmax, b);
-                    cmax[k] = max(cmax[k], b);
-                }
-                rmax = __reduce_max_sync(kFull, rmax);
-                if (lane == 0 && rb + i < r1) atomic_max_nonneg(row_max + rb + i, rmax);
-            }
+        for (int i = 0; i < 4; ++i) {
+            const float4* src = reinterpret_cast<const float4*>(v + static_cast<int64_t>(min(rb + i, r1 - 1)) * cols + c0) + lane;
+            const float4 a = __ldg(src), b = __ldg(src + 32);
+            x[i][0] = a.x; x[i][1] = a.y; x[i][2] = a.z; x[i][3] = a.w;
+            x[i][4] = b.x; x[i][5] = b.y; x[i][6] = b.z; x[i][7] = b.w;
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) atomic_max_nonneg(col_max + c0 + (k < 4 ? 0 : 124) + lane * 4 + k, cmax[k]);
-    } else {
-        const int64_t numel = static_cast<int64_t>(rows) * cols;
-        const int64_t start = item * (kPanelCols * kRowsPerItem);
-        for (int it = 0; it < kRowsPerItem; ++it) {
-            const int64_t e = start + static_cast<int64_t>(it) * kPanelCols + lane * 8;
-            if (e >= numel) break;
-            const int nv = static_cast<int>(min(static_cast<int64_t>(8), numel - e));
-            int64_t r = e / cols;
-            int c = static_cast<int>(e - r * cols);
-            for (int k = 0; k < nv; ++k) {
-                const uint32_t b = absbits(v[e + k]);
-                atomic_max_nonneg(row_max + r, b);
-                atomic_max_nonneg(col_max + c, b);
-                if (++c == cols) {
-                    c = 0;
-                    ++r;
+        for (int i = 0; i < 4; ++i) {
+            uint32_t rmax = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t b = absbits(x[i][k]);
+                rmax = max(rmax, b);
+                cmax[k] = max(cmax[k], b);
+            }
+            rmax = __reduce_max_sync(kFull, rmax);
+            if (lane == 0 && rb + i < r1) atomic_max_nonneg(row_max + rb + i, rmax);
+        }
+    }
+    reinterpret_cast<uint4*>(warp_max[warp])[lane] = make_uint4(cmax[0], cmax[1], cmax[2], cmax[3]);
+    reinterpret_cast<uint4*>(warp_max[warp])[32 + lane] = make_uint4(cmax[4], cmax[5], cmax[6], cmax[7]);
+    __syncthreads();
+    uint32_t c = 0;
+#pragma unroll
+    for (int w = 0; w < kWarpsPerCta; ++w) c = max(c, warp_max[w][threadIdx.x]);
+    atomic_max_nonneg(col_max + c0 + threadIdx.x, c);
+}
+
+// The same for any shape and alignment: one atomic on the row and one on the column per element.
+__global__ void __launch_bounds__(kThreads)
+rank1_max_kernel(const float* __restrict__ v, int rows, int cols, float* __restrict__ row_max, float* __restrict__ col_max) {
+    const int lane = threadIdx.x & 31;
+    const int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
+    const int64_t numel = static_cast<int64_t>(rows) * cols;
+    const int64_t start = item * (kPanelCols * kRowsPerItem);
+    for (int it = 0; it < kRowsPerItem; ++it) {
+        const int64_t e = start + static_cast<int64_t>(it) * kPanelCols + lane * 8;
+        if (e >= numel) break;
+        const int nv = static_cast<int>(min(static_cast<int64_t>(8), numel - e));
+        int64_t r = e / cols;
+        int c = static_cast<int>(e - r * cols);
+        for (int k = 0; k < nv; ++k) {
+            const uint32_t b = absbits(v[e + k]);
+            atomic_max_nonneg(row_max + r, b);
+            atomic_max_nonneg(col_max + c, b);
+            if (++c == cols) {
+                c = 0;
+                ++r;
+            }
+        }
+    }
+}
+
+// ---- strips (see the step kernels): matrices whose rows are no whole panels, buffers vector-aligned, from 8 columns on ----
+// One CTA per strip.  Lane L works on the quads 4L .. 4L+3 and 128+4L .. 128+4L+3 of a run, for the same reason as above.
+struct StripWalk {   // a lane's two quads, a turn of the CTA (2048 elements) at a time
+    StripItem it;
+    int cols, off, r[2], c[2];
+    __device__ __forceinline__ StripWalk(int rows, int cols_, int runs, int64_t li) : cols(cols_) {
+        DevTensor t;
+        t.rows = rows;
+        t.cols = cols_;
+        t.numel = static_cast<int64_t>(rows) * cols_;
+        t.flat_off = 0;
+        t.strip_runs = runs;
+        it = strip_item(t, li);
+        off = static_cast<int>(threadIdx.x >> 5) * kPanelCols + static_cast<int>(threadIdx.x & 31) * 4;
+        for (int h = 0; h < 2; ++h) position(it.e0 + off + h * 128, cols, r[h], c[h]);
+    }
+    __device__ __forceinline__ int first(int h) const { return it.window ? off + h * 128 : c[h]; }
+    __device__ __forceinline__ void advance() {
+        off += kThreads * 8;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            r[h] += it.row_step;
+            c[h] += it.col_step;
+            if (c[h] >= cols) {
+                c[h] -= cols;
+                ++r[h];
+            }
+        }
+    }
+};
+// Elements e .. e+3 of an fp32 array of n elements, zeros behind its end.
+__device__ __forceinline__ float4 load_quad(const float* x, int64_t e, int64_t n) {
+    if (e + 4 <= n) return __ldg(reinterpret_cast<const float4*>(x + e));
+    float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (e < n) q.x = x[e];
+    if (e + 1 < n) q.y = x[e + 1];
+    if (e + 2 < n) q.z = x[e + 2];
+    return q;
+}
+
+__global__ void __launch_bounds__(kThreads)
+rank1_max_strip_kernel(const float* __restrict__ v, int rows, int cols, float* __restrict__ row_max, float* __restrict__ col_max, int runs) {
+    extern __shared__ uint32_t strip_max[];
+    StripWalk w(rows, cols, runs, blockIdx.x);
+    const int64_t numel = static_cast<int64_t>(rows) * cols;
+    const int lane = threadIdx.x & 31;
+    float4 next[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) next[h] = load_quad(v, w.it.e0 + w.off + h * 128, numel);
+    for (int i = threadIdx.x; i < w.it.entries; i += kThreads) strip_max[spread(i)] = 0;
+    __syncthreads();
+    for (int run = 0; run < runs; ++run) {
+        const int64_t e = w.it.e0 + w.off;
+        if (e - lane * 4 >= numel) break;   // warp-uniform
+        float x[2][4];
+        int r[2], left[2], first[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            x[h][0] = next[h].x; x[h][1] = next[h].y; x[h][2] = next[h].z; x[h][3] = next[h].w;
+            r[h] = w.r[h];
+            left[h] = cols - w.c[h];
+            first[h] = w.first(h);
+        }
+        w.advance();
+        if (run + 1 < runs) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) next[h] = load_quad(v, w.it.e0 + w.off + h * 128, numel);
+        }
+        uint32_t m[2][2] = {{0, 0}, {0, 0}};   // of either quad: the part in row r, the part in row r + 1
+        int r_hi = 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t eh = e + h * 128;
+            const int nv = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(4), numel - eh)));
+            if (nv) r_hi = max(r_hi, r[h] + (nv > left[h] ? 1 : 0));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t b = k < nv ? absbits(x[h][k]) : 0u;
+                const bool over = k >= left[h];
+                m[h][0] = max(m[h][0], over ? 0u : b);
+                m[h][1] = max(m[h][1], over ? b : 0u);
+                const int word = strip_word(first[h], k);
+                if (b > strip_max[word]) atomicMax(&strip_max[word], b);
+            }
+        }
+        const int r_lo = __shfl_sync(kFull, r[0], 0);
+        r_hi = __reduce_max_sync(kFull, r_hi);
+        for (int q = r_lo; q <= r_hi; ++q) {
+            uint32_t b = 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) b = max(b, max(r[h] == q ? m[h][0] : 0u, r[h] + 1 == q ? m[h][1] : 0u));
+            b = __reduce_max_sync(kFull, b);
+            if (lane == 0) atomic_max_nonneg(row_max + q, b);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < w.it.entries; i += kThreads) {
+        const uint32_t b = strip_max[spread(i)];
+        if (b) atomic_max_nonneg(col_max + strip_column(w.it, i, cols), b);
+    }
+}
+
+// Quantize / dequantize of a strip against finished maxima.  Quantize walks the strips from the last to the first: what the
+// pass over the maxima has read last is still in L2.
+template <bool QUANT>
+__global__ void __launch_bounds__(kThreads)
+rank1_codec_strip_kernel(const float* __restrict__ in, uint8_t* __restrict__ codes, const float* __restrict__ row_max,
+                         const float* __restrict__ col_max, int rows, int cols, float* __restrict__ out, int runs) {
+    __shared__ SmemPre s;
+    extern __shared__ float strip_col[];
+    load_smem(s);
+    StripWalk w(rows, cols, runs, QUANT ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+    const int64_t numel = static_cast<int64_t>(rows) * cols;
+    const int lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < w.it.entries; i += kThreads) strip_col[spread(i)] = __ldg(col_max + strip_column(w.it, i, cols));
+    __syncthreads();
+    for (int run = 0; run < runs; ++run, w.advance()) {
+        const int64_t e = w.it.e0 + w.off;
+        if (e - lane * 4 >= numel) break;   // warp-uniform
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t eh = e + h * 128;
+            const int nv = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(4), numel - eh)));
+            if (nv == 0) continue;
+            const float row_a = __ldg(row_max + w.r[h]), row_b = __ldg(row_max + min(w.r[h] + 1, rows - 1));
+            const int left = cols - w.c[h], first = w.first(h);
+            float sc[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sc[k] = k < nv ? fminf(k >= left ? row_b : row_a, strip_col[strip_word(first, k)]) : 1.0f;
+            if (QUANT) {
+                const float4 q = load_quad(in, eh, numel);
+                const float x[4] = {q.x, q.y, q.z, q.w};
+                bool ok = true;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) ok &= sc[k] >= 0x1p-90f && sc[k] <= 0x1p100f;
+                uint32_t code = 0;
+                if (ok) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const f2 y = fma2(div2(mk2(x[2 * j], x[2 * j + 1]), mk2(sc[2 * j], sc[2 * j + 1])), bc2(16.0f), bc2(-1.5f));
+                        code += code_from_y(y.x) << (8 * j);
+                        code += code_from_y(y.y) << (8 * j + 4);
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) code |= search16(scaled(x[k], sc[k]), s.t.mv) << (4 * k);
+                }
+                if (nv == 4)
+                    *reinterpret_cast<uint16_t*>(codes + (eh >> 1)) = static_cast<uint16_t>(code);
+                else
+                    store_codes_tail(codes, eh, nv, code & ((1u << (4 * nv)) - 1u));
+            } else {
+                const uint32_t code = nv == 4 ? *reinterpret_cast<const uint16_t*>(codes + (eh >> 1)) : load_codes_tail(codes, eh, nv);
+                const f2 a = mul2(s.qv2.v[code & 0xffu], mk2(sc[0], sc[1])), b = mul2(s.qv2.v[code >> 8 & 0xffu], mk2(sc[2], sc[3]));
+                if (nv == 4) {
+                    *reinterpret_cast<float4*>(out + eh) = make_float4(a.x, a.y, b.x, b.y);
+                } else {
+                    out[eh] = a.x;
+                    if (nv > 1) out[eh + 1] = a.y;
+                    if (nv > 2) out[eh + 2] = b.x;
                 }
             }
         }
@@ -1897,18 +2076,19 @@ rank1_max_kernel(const float* __restrict__ v, int rows, int cols, float* __restr
 // division and the closed-form search where the scales allow it.
 __global__ void __launch_bounds__(kThreads)
 rank1_quant_panel_kernel(const float* __restrict__ in, uint8_t* __restrict__ codes, const float* __restrict__ row_max,
-                         const float* __restrict__ col_max, int rows, int cols) {
+                         const float* __restrict__ col_max, int rows, int cols, int item_rows) {
     __shared__ SmemPre s;
     load_smem(s);
     const int lane = threadIdx.x & 31;
     const int panels = cols / kPanelCols;
-    const int64_t total = static_cast<int64_t>((rows + kRowsPerItem - 1) / kRowsPerItem) * panels;
+    const int64_t total = static_cast<int64_t>((rows + item_rows - 1) / item_rows) * panels;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
-    for (int64_t item = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5); item < total; item += stride) {
+    for (int64_t turn = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5); turn < total; turn += stride) {
+        const int64_t item = total - 1 - turn;   // last item first: what the pass over the maxima has read last is still in L2
         const int band = static_cast<int>(item / panels);
         // lane L takes columns 4L .. 4L+3 and 128+4L .. 128+4L+3 of the panel (512 contiguous bytes per load instruction)
         const int c0 = static_cast<int>(item - static_cast<int64_t>(band) * panels) * kPanelCols;
-        const int r0 = band * kRowsPerItem, r1 = min(r0 + kRowsPerItem, rows);
+        const int r0 = band * item_rows, r1 = min(r0 + item_rows, rows);
         float col[8];
         {
             const float4 a = __ldg(reinterpret_cast<const float4*>(col_max + c0) + lane), b = __ldg(reinterpret_cast<const float4*>(col_max + c0 + 128) + lane);

@@ -65,3 +65,28 @@ def test_matrices_whose_rows_are_no_whole_panels(shape, dtype):
 def test_strips_flat_items_and_panels_in_one_launch():
     run([((300, 300), torch.bfloat16), ((500,), torch.bfloat16), ((64, 512), torch.bfloat16), ((77, 333), torch.float16),
          ((9001,), torch.float32), ((1200, 1500), torch.float32)], dead_rows=0.2)
+
+
+@pytest.mark.parametrize("shape", [(1000, 7), (1000, 8), (1001, 9), (600, 77), (100, 255), (65, 257), (31, 2049), (9, 8191), (9, 8193), (5, 20001),
+                                   (1, 9000), (129, 256), (513, 768), (2, 5)])
+def test_quantize_and_dequantize_matrices_of_any_row_length(shape):
+    import quantfour_adamw_cuda_b200 as qf
+    v = torch.rand(shape) ** 4
+    v[torch.rand(shape[0]) < 0.1] = 0.0          # rows of zeros
+    v.view(-1)[::37] *= 1e-30                    # scales and values outside the range of the fast division
+    codes, row, col = qf.quantize_v(v.to(DEV))
+    want_codes, want_row, want_col = TO.quantize_rank1(v)
+    assert torch.equal(row.cpu(), want_row) and torch.equal(col.cpu(), want_col)
+    assert torch.equal(codes.cpu().view(torch.uint8), want_codes)
+    assert torch.equal(qf.dequantize_v(codes, row, col).cpu(), TO.dequantize_rank1(want_codes, want_row, want_col, *shape))
+
+
+@pytest.mark.parametrize("n", [255, 256, 1025, 4096, 4097, 70_000, 2_000_001])
+@pytest.mark.parametrize("mid,qmap,quantize,dequantize", [("MM", "QM", "quantize_m", "dequantize_m"), ("MV", "QV", "quantize_v_block", "dequantize_v_block")])
+def test_quantize_and_dequantize_blocks_of_short_items(n, mid, qmap, quantize, dequantize):
+    import quantfour_adamw_cuda_b200.functional as F
+    x = torch.randn(n) if mid == "MM" else torch.rand(n)
+    codes, scales = getattr(F, quantize)(x.to(DEV))
+    want_codes, want_scales = TO.quantize_block(x, getattr(TO, mid))
+    assert torch.equal(codes.cpu().view(torch.uint8), want_codes) and torch.equal(scales.cpu(), want_scales)
+    assert torch.equal(getattr(F, dequantize)(codes, scales, n).cpu(), TO.dequantize_block(want_codes, want_scales, n, getattr(TO, qmap)))
