@@ -99,9 +99,7 @@ struct Plan {
     int n = 0;                    // tensors in the table (zero-size tensors dropped)
     int64_t items[kTables] = {};
     int n_rank1 = 0;
-    bool any_f32_panel = false;   // sizes the staging ring of the panel kernel
-    bool any_bf16_panel = false;
-    bool any_f16_panel = false;
+    bool f32[3] = {}, bf16[3] = {}, f16[3] = {};   // whether a mapping (qf::kMap..) has tensors of a dtype
     qf::DevTensor* d_tensors = nullptr;
     int64_t* d_base[kTables] = {};
     uint32_t* d_status = nullptr;
@@ -218,9 +216,6 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
             if (panel) {
                 t.flags |= qf::kFlagPanel;
                 t.panels = static_cast<int32_t>(d.cols / qf::kPanelCols);
-                if (d.dtype == QF_F32) plan->any_f32_panel = true;
-                if (d.dtype == QF_BF16) plan->any_bf16_panel = true;
-                if (d.dtype == QF_F16) plan->any_f16_panel = true;
             } else if (strip_fits(d.cols, vec)) {
                 t.flags |= qf::kFlagStrip;
             }
@@ -228,6 +223,8 @@ int build_plan(const QfTensorDesc* descs, int n_tensors, int n_hypers, void* wor
         }
         if (vec) t.flags |= qf::kFlagVec;
         const bool panel = t.flags & qf::kFlagPanel, strip = t.flags & qf::kFlagStrip;
+        const int map = panel ? qf::kMapPanel : strip ? qf::kMapStrip : qf::kMapFlat;
+        (d.dtype == QF_F32 ? plan->f32 : d.dtype == QF_BF16 ? plan->bf16 : plan->f16)[map] = true;
         if (panel)
             panel_rows += d.rows * t.panels;
         else
@@ -318,6 +315,7 @@ int sm_count() {
     return cached[dev];
 }
 constexpr int kGridWaves = 16;
+constexpr int kMergeRounds = 4;
 unsigned persistent_grid(int64_t items, int per_sm, int waves = kGridWaves) {
     const int64_t ctas = (items + qf::kWarpsPerCta - 1) / qf::kWarpsPerCta;
     const int64_t cap = static_cast<int64_t>(sm_count()) * per_sm * waves;
@@ -370,29 +368,52 @@ qf::Sched no_sched() {
     return sc;
 }
 
-unsigned cta_grid(int64_t items, int per_sm) {   // one item per CTA and turn
-    return static_cast<unsigned>(std::min<int64_t>(items, static_cast<int64_t>(sm_count()) * per_sm * kGridWaves));
+// The part of a launch that serves one mapping, or nothing.
+qf::Work work_of(const Plan& pl) {
+    qf::Work w;
+    memset(&w, 0, sizeof w);
+    w.n = pl.n;
+    return w;
+}
+void add_part(qf::Work* w, const Plan& pl, int map, int table, int64_t ctas, int per_sm) {
+    w->base[map] = pl.d_base[table];
+    w->ctas[map] = static_cast<int32_t>(std::min<int64_t>(ctas, static_cast<int64_t>(sm_count()) * per_sm * kGridWaves));
+}
+unsigned ctas_of(const qf::Work& w) { return static_cast<unsigned>(w.ctas[0]) + w.ctas[1] + w.ctas[2]; }
+// Whether the mappings of a pass go into one launch: where there is more than one and the launch is a few rounds of the
+// device, its launches and their ends are what counts (a transformer layer of width 1024: see step_main_kernel); from
+// there on a kernel for the panels alone, whose loop is scheduled a little better, is worth a launch of its own.
+bool merge_parts(const qf::Work& w, int per_sm) {
+    const int parts = (w.ctas[0] > 0) + (w.ctas[1] > 0) + (w.ctas[2] > 0);
+    return parts > 1 && ctas_of(w) <= static_cast<unsigned>(sm_count()) * per_sm * kMergeRounds;
+}
+qf::Work only(qf::Work w, int map) {
+    for (int k = 0; k < 3; ++k)
+        if (k != map) w.ctas[k] = 0;
+    return w;
 }
 
+// One launch of the first pass.
+template <int MAP, bool SCALE, bool SCHED>
+int launch_pre_map(const Plan& pl, const qf::Work& w, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
+    const int panel_smem = w.ctas[qf::kMapPanel] ? qf::pre_dyn_smem(pl.f32[qf::kMapPanel]) : 0;
+    const int smem = std::max(panel_smem, w.ctas[qf::kMapStrip] ? qf::strip_dyn_smem() : 0);
+    return launch_chained<qf::step_pre_kernel<MAP, SCALE, SCHED>>(ctas_of(w), smem, std::max(qf::pre_dyn_smem(true), qf::strip_dyn_smem()), stream,
+                                                                pl.d_tensors, w, hp, panel_smem / qf::kWarpsPerCta, pl.d_status, sc);
+}
 template <bool SCALE, bool SCHED>
-int launch_pre_panel(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
-    const int dyn = qf::pre_dyn_smem(pl.any_f32_panel);
-    return launch_chained<qf::step_pre_kernel<qf::kMapPanel, SCALE, SCHED>>(
-        cta_grid(pl.items[kPrePanel], qf::kPreMinCtas), dyn, qf::pre_dyn_smem(true), stream, pl.d_tensors, pl.d_base[kPrePanel], pl.n, hp,
-        dyn / qf::kWarpsPerCta, pl.d_status, sc);
-}
-
-// First pass over the strips and over the flat items; the kernels see by themselves whether a gradient scale is set.
-template <bool SCHED>
-int launch_pre_others(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
-    if (pl.items[kStrip])
-        if (int rc = launch_chained<qf::step_pre_kernel<qf::kMapStrip, false, SCHED>>(
-                cta_grid(pl.items[kStrip], qf::kPreMinCtas), qf::strip_dyn_smem(), qf::strip_dyn_smem(), stream, pl.d_tensors,
-                pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, sc))
-            return rc;
-    if (pl.items[kPreFlat])
-        return launch_chained<qf::step_pre_kernel<qf::kMapFlat, false, SCHED>>(
-            persistent_grid(pl.items[kPreFlat], qf::kPreMinCtas), 0, 0, stream, pl.d_tensors, pl.d_base[kPreFlat], pl.n, hp, 0, pl.d_status, sc);
+int launch_pre_all(const Plan& pl, const qf::HyperPack& hp, const qf::Sched& sc, cudaStream_t stream) {
+    qf::Work w = work_of(pl);
+    add_part(&w, pl, qf::kMapPanel, kPrePanel, pl.items[kPrePanel], qf::kPreMinCtas);
+    add_part(&w, pl, qf::kMapStrip, kStrip, pl.items[kStrip], qf::kPreMinCtas);
+    add_part(&w, pl, qf::kMapFlat, kPreFlat, ceil_div(pl.items[kPreFlat], qf::kWarpsPerCta), qf::kPreMinCtas);
+    if (!SCHED && merge_parts(w, qf::kPreMinCtas)) return launch_pre_map<qf::kMapAll, SCALE, false>(pl, w, hp, sc, stream);
+    // strips and flat items look at the scale by themselves
+    if (w.ctas[qf::kMapPanel])
+        if (int rc = launch_pre_map<qf::kMapPanel, SCALE, SCHED>(pl, only(w, qf::kMapPanel), hp, sc, stream)) return rc;
+    if (w.ctas[qf::kMapStrip])
+        if (int rc = launch_pre_map<qf::kMapStrip, false, SCHED>(pl, only(w, qf::kMapStrip), hp, sc, stream)) return rc;
+    if (w.ctas[qf::kMapFlat]) return launch_pre_map<qf::kMapFlat, false, SCHED>(pl, only(w, qf::kMapFlat), hp, sc, stream);
     return QF_OK;
 }
 
@@ -403,77 +424,77 @@ int launch_pre(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStream
                bool scaled = false) {
     if (pl.n_rank1 == 0) return QF_OK;
     if (int rc = roll(pl, qf::kRollClear | (keep ? qf::kRollKeep : 0), stream)) return rc;
-    if (pl.items[kPrePanel]) {
-        // the variant that rewrites the gradients runs only when some set asks for it
-        if (!sched)
-            for (int k = 0; k < n_hypers; ++k) scaled = scaled || hp.h[k].gs != 1.0f;
-        int rc;
-        if (sched)
-            rc = scaled ? launch_pre_panel<true, true>(pl, hp, *sched, stream) : launch_pre_panel<false, true>(pl, hp, *sched, stream);
-        else
-            rc = scaled ? launch_pre_panel<true, false>(pl, hp, no_sched(), stream) : launch_pre_panel<false, false>(pl, hp, no_sched(), stream);
-        if (rc) return rc;
-    }
-    if (int rc = sched ? launch_pre_others<true>(pl, hp, *sched, stream) : launch_pre_others<false>(pl, hp, no_sched(), stream)) return rc;
-    QF_CUDA(cudaGetLastError());
-    return QF_OK;
+    // the variant that rewrites the gradients runs only when some set asks for it
+    if (sched)
+        return scaled ? launch_pre_all<true, true>(pl, hp, *sched, stream) : launch_pre_all<false, true>(pl, hp, *sched, stream);
+    for (int k = 0; k < n_hypers; ++k) scaled = scaled || hp.h[k].gs != 1.0f;
+    return scaled ? launch_pre_all<true, false>(pl, hp, no_sched(), stream) : launch_pre_all<false, false>(pl, hp, no_sched(), stream);
 }
 
-template <bool PUSH, bool BC1, bool SCHED, bool RELAXED, int DT>
-int launch_main_panel_dt(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, cudaStream_t stream) {
-    const int dyn = qf::main_dyn_smem(pl.any_f32_panel);
-    const int ring = qf::kStages * (pl.any_f32_panel ? qf::kRowBytesF32 : qf::kRowBytesBf16);
-    return launch_chained<qf::step_main_kernel<qf::kMapPanel, PUSH, BC1, SCHED, RELAXED, DT>>(
-        persistent_grid(pl.items[kMainPanel], qf::kMainMinCtas), dyn, qf::main_dyn_smem(true), stream, pl.d_tensors, pl.d_base[kMainPanel],
-        pl.n, hp, ring, pl.d_status, pp, sc, pl.d_base[kRoll], static_cast<int>(pl.items[kRoll]));
+// One launch of the second pass; `rolls`: the items of row and column maxima it stores.
+template <int MAP, bool PUSH, bool BC1, bool SCHED, bool RELAXED, int DT>
+int launch_main_dt(const Plan& pl, const qf::Work& w, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, int rolls,
+                   cudaStream_t stream) {
+    const bool f32 = pl.f32[qf::kMapPanel];
+    const int panel_smem = w.ctas[qf::kMapPanel] ? qf::main_dyn_smem(f32) : 0;
+    const int smem = std::max(panel_smem, w.ctas[qf::kMapStrip] ? qf::strip_dyn_smem() : 0);
+    const int ring = qf::kStages * (f32 ? qf::kRowBytesF32 : qf::kRowBytesBf16);
+    return launch_chained<qf::step_main_kernel<MAP, PUSH, BC1, SCHED, RELAXED, DT>>(
+        ctas_of(w), smem, std::max(qf::main_dyn_smem(true), qf::strip_dyn_smem()), stream, pl.d_tensors, w, hp, ring, pl.d_status, pp, sc,
+        pl.d_base[kRoll], rolls);
 }
-// A launch whose panel tensors are all of one dtype takes the kernel that carries that dtype's loop only (the plain
-// step, the common case; the rarer variants keep the two-dtype kernel): 1.4 % faster, measured.
-template <bool PUSH, bool BC1, bool SCHED, bool RELAXED = false>
-int launch_main_panel(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, cudaStream_t stream) {
+// A launch whose tensors are all of one dtype takes the kernel that carries that dtype's loops only (the plain
+// step, the common case; the rarer variants keep the kernel of all dtypes): 1.4 % faster on panels, measured.
+template <int MAP, bool PUSH, bool BC1, bool SCHED, bool RELAXED = false>
+int launch_main_map(const Plan& pl, const qf::Work& w, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, int rolls,
+                    cudaStream_t stream) {
     if (!PUSH && !SCHED && !RELAXED) {
-        if (!pl.any_f32_panel && !pl.any_f16_panel) return launch_main_panel_dt<false, BC1, false, false, 1>(pl, hp, pp, sc, stream);
-        if (!pl.any_bf16_panel && !pl.any_f16_panel) return launch_main_panel_dt<false, BC1, false, false, 2>(pl, hp, pp, sc, stream);
-        if (!pl.any_bf16_panel && !pl.any_f32_panel) return launch_main_panel_dt<false, BC1, false, false, 3>(pl, hp, pp, sc, stream);
+        bool f32 = false, bf16 = false, f16 = false;
+        for (int map = 0; map < 3; ++map) {
+            if (!w.ctas[map]) continue;
+            f32 = f32 || pl.f32[map];
+            bf16 = bf16 || pl.bf16[map];
+            f16 = f16 || pl.f16[map];
+        }
+        if (!f32 && !f16) return launch_main_dt<MAP, false, BC1, false, false, 1>(pl, w, hp, pp, sc, rolls, stream);
+        if (!bf16 && !f16) return launch_main_dt<MAP, false, BC1, false, false, 2>(pl, w, hp, pp, sc, rolls, stream);
+        if (!bf16 && !f32) return launch_main_dt<MAP, false, BC1, false, false, 3>(pl, w, hp, pp, sc, rolls, stream);
     }
-    return launch_main_panel_dt<PUSH, BC1, SCHED, RELAXED, 0>(pl, hp, pp, sc, stream);
-}
-
-// Second pass over the strips and over the flat items.  The new maxima are stored by the first launch of the pass.
-template <bool PUSH, bool SCHED>
-int launch_main_others(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, cudaStream_t stream) {
-    int rolls = pl.items[kMainPanel] ? 0 : static_cast<int>(pl.items[kRoll]);
-    if (pl.items[kStrip]) {
-        if (int rc = launch_chained<qf::step_main_kernel<qf::kMapStrip, PUSH, false, SCHED>>(
-                cta_grid(pl.items[kStrip], qf::kMainMinCtas), qf::strip_dyn_smem(), qf::strip_dyn_smem(), stream, pl.d_tensors,
-                pl.d_base[kStrip], pl.n, hp, 0, pl.d_status, pp, sc, pl.d_base[kRoll], rolls))
-            return rc;
-        rolls = 0;
-    }
-    if (pl.items[kMainFlat])
-        return launch_chained<qf::step_main_kernel<qf::kMapFlat, PUSH, false, SCHED>>(
-            persistent_grid(pl.items[kMainFlat], qf::kMainMinCtas), 0, 0, stream, pl.d_tensors, pl.d_base[kMainFlat], pl.n, hp, 0, pl.d_status,
-            pp, sc, pl.d_base[kRoll], rolls);
-    return QF_OK;
+    return launch_main_dt<MAP, PUSH, BC1, SCHED, RELAXED, 0>(pl, w, hp, pp, sc, rolls, stream);
 }
 
 // bc_one: every hyper-parameter set of the call has bc2s == 1 exactly (late in a run): the panel kernel then
 // runs the variant without the division by it.
 // relaxed (without peer stores only): the panel kernel whose bf16 parameter update is uncorrected.
-template <bool PUSH>
-int launch_main_kernels(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, bool bc_one, cudaStream_t stream,
-                        bool relaxed = false) {
-    if (pl.items[kMainPanel]) {
+template <bool PUSH, bool SCHED>
+int launch_main_all(const Plan& pl, const qf::HyperPack& hp, const qf::PushPack& pp, const qf::Sched& sc, bool bc_one, bool relaxed,
+                    cudaStream_t stream) {
+    qf::Work w = work_of(pl);
+    add_part(&w, pl, qf::kMapPanel, kMainPanel, ceil_div(pl.items[kMainPanel], qf::kWarpsPerCta), qf::kMainMinCtas);
+    add_part(&w, pl, qf::kMapStrip, kStrip, pl.items[kStrip], qf::kMainMinCtas);
+    add_part(&w, pl, qf::kMapFlat, kMainFlat, ceil_div(pl.items[kMainFlat], qf::kWarpsPerCta), qf::kMainMinCtas);
+    int rolls = static_cast<int>(pl.items[kRoll]);   // stored by the first launch of the pass
+    if (!PUSH && !SCHED && !relaxed && merge_parts(w, qf::kMainMinCtas))
+        return launch_main_map<qf::kMapAll, false, false, false>(pl, w, hp, pp, sc, rolls, stream);
+    if (w.ctas[qf::kMapPanel]) {
+        const qf::Work panels = only(w, qf::kMapPanel);
         int rc;
-        if (!PUSH && relaxed)
-            rc = bc_one ? launch_main_panel<false, true, false, true>(pl, hp, pp, no_sched(), stream)
-                        : launch_main_panel<false, false, false, true>(pl, hp, pp, no_sched(), stream);
+        if (!PUSH && !SCHED && relaxed)
+            rc = bc_one ? launch_main_map<qf::kMapPanel, false, true, false, true>(pl, panels, hp, pp, sc, rolls, stream)
+                        : launch_main_map<qf::kMapPanel, false, false, false, true>(pl, panels, hp, pp, sc, rolls, stream);
+        else if (!SCHED && bc_one)
+            rc = launch_main_map<qf::kMapPanel, PUSH, true, false>(pl, panels, hp, pp, sc, rolls, stream);
         else
-            rc = bc_one ? launch_main_panel<PUSH, true, false>(pl, hp, pp, no_sched(), stream)
-                        : launch_main_panel<PUSH, false, false>(pl, hp, pp, no_sched(), stream);
+            rc = launch_main_map<qf::kMapPanel, PUSH, false, SCHED>(pl, panels, hp, pp, sc, rolls, stream);
         if (rc) return rc;
+        rolls = 0;
     }
-    return launch_main_others<PUSH, false>(pl, hp, pp, no_sched(), stream);
+    if (w.ctas[qf::kMapStrip]) {
+        if (int rc = launch_main_map<qf::kMapStrip, PUSH, false, SCHED>(pl, only(w, qf::kMapStrip), hp, pp, sc, rolls, stream)) return rc;
+        rolls = 0;
+    }
+    if (w.ctas[qf::kMapFlat]) return launch_main_map<qf::kMapFlat, PUSH, false, SCHED>(pl, only(w, qf::kMapFlat), hp, pp, sc, rolls, stream);
+    return QF_OK;
 }
 
 // `push`: null, or the peer copies of the parameter buffer the kernels also store into.
@@ -489,17 +510,9 @@ int launch_main(const Plan& pl, const qf::HyperPack& hp, int n_hypers, cudaStrea
     for (int k = 0; k < n_hypers; ++k) bc_one = bc_one && hp.h[k].fast && hp.h[k].h.bc2s == 1.0f;
     qf::PushPack none;
     memset(&none, 0, sizeof none);
-    if (sched) {
-        if (pl.items[kMainPanel])
-            if (int rc = launch_main_panel<false, false, true>(pl, hp, none, *sched, stream)) return rc;
-        if (int rc = launch_main_others<false, true>(pl, hp, none, *sched, stream)) return rc;
-    } else if (push && push->n > 0) {
-        if (int rc = launch_main_kernels<true>(pl, hp, *push, bc_one, stream)) return rc;
-    } else {
-        if (int rc = launch_main_kernels<false>(pl, hp, none, bc_one, stream, relaxed)) return rc;
-    }
-    QF_CUDA(cudaGetLastError());
-    return QF_OK;
+    if (sched) return launch_main_all<false, true>(pl, hp, none, *sched, false, false, stream);
+    if (push && push->n > 0) return launch_main_all<true, false>(pl, hp, *push, no_sched(), bc_one, false, stream);
+    return launch_main_all<false, false>(pl, hp, none, no_sched(), bc_one, relaxed, stream);
 }
 
 using qf::widen_hyper;
@@ -1069,9 +1082,7 @@ int qf_step_rank1_noalloc(void* p, const void* g, void* m_codes, void* v_codes, 
     Plan pl;
     pl.n = 1;
     pl.n_rank1 = 1;
-    pl.any_f32_panel = panel && dtype == QF_F32;
-    pl.any_bf16_panel = panel && dtype == QF_BF16;
-    pl.any_f16_panel = panel && dtype == QF_F16;
+    (dtype == QF_F32 ? pl.f32 : dtype == QF_BF16 ? pl.bf16 : pl.f16)[panel ? qf::kMapPanel : strip ? qf::kMapStrip : qf::kMapFlat] = true;
     pl.d_status = reinterpret_cast<uint32_t*>(scratch);
     pl.d_tensors = reinterpret_cast<qf::DevTensor*>(scratch + offsetof(Header, t));
     for (int k = 0; k < kTables; ++k) {

@@ -1447,21 +1447,51 @@ rank1_roll_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restri
 }
 
 // =================================================================================================
-// Multi-tensor kernels.  `base` is the prefix-sum table of the mapping the kernel serves; tensors of
-// the other mapping have zero items in it.
+// Multi-tensor kernels
 // =================================================================================================
 
-// The multi-tensor kernels are persistent: the host launches about as many CTAs as fit on the device and every
-// warp walks the item list with a fixed stride, so the shared-memory tables are filled once per CTA.
-enum { kMapFlat = 0, kMapPanel = 1, kMapStrip = 2 };   // MAP: the mapping a kernel serves
+// The multi-tensor kernels are persistent: the host launches up to a few times as many CTAs as fit on the device and they
+// walk the item lists of their mapping with a fixed stride.
+enum { kMapFlat = 0, kMapPanel = 1, kMapStrip = 2, kMapAll = 3 };   // MAP: the mapping a kernel serves; kMapAll: each CTA
+                                                                     // one of the three, by its number
+// What a launch works on: per mapping the prefix-sum table of its items and the number of CTAs that walk it (tensors of
+// the other mappings have zero items in a table).
+struct Work {
+    const int64_t* base[3];
+    int32_t ctas[3];
+    int32_t n;   // tensors
+};
+// The mapping this CTA serves, and its number among the CTAs that do.
+template <int MAP>
+__device__ __forceinline__ int part_of(const Work& w, int& part) {
+    part = blockIdx.x;
+    if (MAP != kMapAll) return MAP;
+    if (part < w.ctas[kMapPanel]) return kMapPanel;
+    part -= w.ctas[kMapPanel];
+    if (part < w.ctas[kMapStrip]) return kMapStrip;
+    part -= w.ctas[kMapStrip];
+    return kMapFlat;
+}
+// fn(tensor index, item of that tensor) for every item of this CTA (PER_WARP: of this warp).
+template <bool PER_WARP, typename Fn>
+__device__ __forceinline__ void for_items(const Work& w, int map, int part, Fn fn) {
+    const int64_t* __restrict__ base = w.base[map];
+    const int per_cta = PER_WARP ? kWarpsPerCta : 1;
+    const int64_t total = base[w.n], stride = static_cast<int64_t>(w.ctas[map]) * per_cta;
+    for (int64_t item = static_cast<int64_t>(part) * per_cta + (PER_WARP ? threadIdx.x >> 5 : 0); item < total; item += stride) {
+        const int ti = find_tensor(base, w.n, item);
+        fn(ti, item - base[ti]);
+    }
+}
+
 constexpr int kPreMinCtas = 3;   // CTAs per SM the first pass is compiled for (80 registers)
 // SCALE (panel mapping): some hyper-parameter set of the launch carries a gradient scale other than 1.
 // SCHED: the hyper-parameter sets come from the device-resident table `sc` instead of `hp`.
 // (Forms of this kernel that carry one dtype's loop only, as step_main_kernel has them, measured 5 % slower.)
 template <int MAP, bool SCALE = false, bool SCHED = false>
 __global__ void __launch_bounds__(kThreads, kPreMinCtas)
-step_pre_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict__ base, int n,
-                const __grid_constant__ HyperPack hp, int ring_bytes, uint32_t* status, const __grid_constant__ Sched sc) {
+step_pre_kernel(const DevTensor* __restrict__ tensors, const __grid_constant__ Work w, const __grid_constant__ HyperPack hp, int ring_bytes,
+                uint32_t* status, const __grid_constant__ Sched sc) {
     __shared__ SmemPre s;
     __shared__ HyperDev sched_h[SCHED ? QF_MAX_HYPERS : 1];
     dependents_may_launch();
@@ -1471,38 +1501,47 @@ step_pre_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict
         load_sched(sched_h, sc);
         __syncthreads();
     }
-    extern __shared__ __align__(16) char staging[];  // panel kernel: one ring of rows per warp
-    char* stage = staging + (threadIdx.x >> 5) * ring_bytes;
-    const int64_t total = base[n], per_cta = MAP == kMapFlat ? kWarpsPerCta : 1, stride = gridDim.x * per_cta;
-    for (int64_t item = blockIdx.x * per_cta + (MAP == kMapFlat ? threadIdx.x >> 5 : 0); item < total; item += stride) {
-        const int ti = find_tensor(base, n, item);
-        const DevTensor t = tensors[ti];
-        const int64_t li = item - base[ti];
-        const HyperDev& h = SCHED ? sched_h[t.hyper] : hp.h[t.hyper];
-        if (MAP == kMapStrip) {
-            float* words = reinterpret_cast<float*>(staging);
-            uint32_t* col_max = reinterpret_cast<uint32_t*>(words + kStripWords);
-            if (t.dtype == QF_BF16)
-                pre_strip<__nv_bfloat16>(t, li, h, s, words, col_max, status);
-            else if (t.dtype == QF_F16)
-                pre_strip<__half>(t, li, h, s, words, col_max, status);
-            else
-                pre_strip<float>(t, li, h, s, words, col_max, status);
-        } else if (MAP == kMapPanel) {
+    extern __shared__ __align__(16) char staging[];  // panels: one ring of rows per warp; strips: the column scalars
+    int part;
+    const int map = part_of<MAP>(w, part);
+    if ((MAP == kMapPanel || MAP == kMapAll) && map == kMapPanel) {
+        char* stage = staging + (threadIdx.x >> 5) * ring_bytes;
+        for_items<false>(w, kMapPanel, part, [&](int ti, int64_t li) {
+            const DevTensor t = tensors[ti];
+            const HyperDev& h = SCHED ? sched_h[t.hyper] : hp.h[t.hyper];
             if (t.dtype == QF_BF16)
                 pre_panel<__nv_bfloat16, SCALE>(t, li, h, s, stage, ring_bytes, status);
             else if (t.dtype == QF_F16)
                 pre_panel<__half, SCALE>(t, li, h, s, stage, ring_bytes, status);
             else
                 pre_panel<float, SCALE>(t, li, h, s, stage, ring_bytes, status);
-        } else {
+        });
+    }
+    if ((MAP == kMapStrip || MAP == kMapAll) && map == kMapStrip) {
+        float* words = reinterpret_cast<float*>(staging);
+        uint32_t* col_max = reinterpret_cast<uint32_t*>(words + kStripWords);
+        for_items<false>(w, kMapStrip, part, [&](int ti, int64_t li) {
+            const DevTensor t = tensors[ti];
+            const HyperDev& h = SCHED ? sched_h[t.hyper] : hp.h[t.hyper];
+            if (t.dtype == QF_BF16)
+                pre_strip<__nv_bfloat16>(t, li, h, s, words, col_max, status);
+            else if (t.dtype == QF_F16)
+                pre_strip<__half>(t, li, h, s, words, col_max, status);
+            else
+                pre_strip<float>(t, li, h, s, words, col_max, status);
+        });
+    }
+    if ((MAP == kMapFlat || MAP == kMapAll) && map == kMapFlat) {
+        for_items<true>(w, kMapFlat, part, [&](int ti, int64_t li) {
+            const DevTensor t = tensors[ti];
+            const HyperDev& h = SCHED ? sched_h[t.hyper] : hp.h[t.hyper];
             if (t.dtype == QF_BF16)
                 pre_flat_rank1<__nv_bfloat16>(t, li, h, s, status);
             else if (t.dtype == QF_F16)
                 pre_flat_rank1<__half>(t, li, h, s, status);
             else
                 pre_flat_rank1<float>(t, li, h, s, status);
-        }
+        });
     }
 }
 
@@ -1523,15 +1562,15 @@ constexpr int kMainMinCtas = 2;  // CTAs per SM the second pass is compiled for 
 // BC1 (panel mapping only): every hyper-parameter set of the launch has bc2s == 1.
 // SCHED: the hyper-parameter sets come from the device-resident table `sc` instead of `hp`.
 // RELAXED (panel mapping, bf16 tensors): the uncorrected parameter update of adamw_pair_panel.
-// DT (panel mapping): 0 = tensors of several dtypes, 1 = the launch holds bf16 panel tensors only, 2 = fp32 only, 3 = fp16
-// only; a kernel that carries one dtype's loop is scheduled a little better than one that carries all.
+// DT: 0 = tensors of several dtypes, 1 = the launch works on bf16 tensors only, 2 = fp32 only, 3 = fp16 only; a kernel that
+// carries one dtype's loops is scheduled a little better than one that carries all.
 // Every CTA ends with its share of the `n_roll` items that store the new row / column maxima (kRollCommit): the second
 // pass reads the old ones from the copies, so nothing has to wait for them.
 template <int MAP, bool PUSH, bool BC1 = false, bool SCHED = false, bool RELAXED = false, int DT = 0>
 __global__ void __launch_bounds__(kThreads, kMainMinCtas)
-step_main_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restrict__ base, int n,
-                 const __grid_constant__ HyperPack hp, int ring_bytes, uint32_t* status,
-                 const __grid_constant__ PushPack pp, const __grid_constant__ Sched sc, const int64_t* __restrict__ roll_base, int n_roll) {
+step_main_kernel(const DevTensor* __restrict__ tensors, const __grid_constant__ Work w, const __grid_constant__ HyperPack hp, int ring_bytes,
+                 uint32_t* status, const __grid_constant__ PushPack pp, const __grid_constant__ Sched sc,
+                 const int64_t* __restrict__ roll_base, int n_roll) {
     const PushPack* push = PUSH ? &pp : nullptr;
     __shared__ Smem s;
     __shared__ HyperDev sched_h[SCHED ? QF_MAX_HYPERS : 1];
@@ -1542,39 +1581,48 @@ step_main_kernel(const DevTensor* __restrict__ tensors, const int64_t* __restric
         load_sched(sched_h, sc);
         __syncthreads();
     }
-    extern __shared__ __align__(16) char staging[];  // panel kernel: per warp a ring of rows plus the column block
-    char* stage = staging + (threadIdx.x >> 5) * (ring_bytes + kColBytes + kRowBufBytes);
-    const int64_t total = base[n], per_cta = MAP == kMapStrip ? 1 : kWarpsPerCta, stride = gridDim.x * per_cta;
-    for (int64_t item = blockIdx.x * per_cta + (MAP == kMapStrip ? 0 : threadIdx.x >> 5); item < total; item += stride) {
-        const int ti = find_tensor(base, n, item);
-        const DevTensor* tp = tensors + ti;
-        const int64_t li = item - base[ti];
-        const HyperDev& h = SCHED ? sched_h[tp->hyper] : hp.h[tp->hyper];  // hp is a grid constant: its address is usable as it is
-        if (MAP == kMapStrip) {
-            float* words = reinterpret_cast<float*>(staging);
-            if (tp->dtype == QF_BF16)
-                main_strip<__nv_bfloat16, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
-            else if (tp->dtype == QF_F16)
-                main_strip<__half, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
-            else
-                main_strip<float, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
-        } else if (MAP == kMapPanel) {
+    extern __shared__ __align__(16) char staging[];  // panels: per warp a ring of rows, the columns, the rows; strips: the column scalars
+    int part;
+    const int map = part_of<MAP>(w, part);
+    if ((MAP == kMapPanel || MAP == kMapAll) && map == kMapPanel) {
+        char* stage = staging + (threadIdx.x >> 5) * (ring_bytes + kColBytes + kRowBufBytes);
+        for_items<true>(w, kMapPanel, part, [&](int ti, int64_t li) {
+            const DevTensor* tp = tensors + ti;
+            const HyperDev& h = SCHED ? sched_h[tp->hyper] : hp.h[tp->hyper];  // hp is a grid constant: its address is usable as it is
             if (DT == 1 || (DT == 0 && tp->dtype == QF_BF16))
                 main_panel<__nv_bfloat16, PUSH, BC1, RELAXED>(tp, li, h, s, stage, ring_bytes, status, push);
             else if (DT == 3 || (DT == 0 && tp->dtype == QF_F16))
                 main_panel<__half, PUSH, BC1>(tp, li, h, s, stage, ring_bytes, status, push);
             else
                 main_panel<float, PUSH, BC1>(tp, li, h, s, stage, ring_bytes, status, push);
-        } else {
-            if (tp->dtype == QF_BF16)
+        });
+    }
+    if ((MAP == kMapStrip || MAP == kMapAll) && map == kMapStrip) {
+        float* words = reinterpret_cast<float*>(staging);
+        for_items<false>(w, kMapStrip, part, [&](int ti, int64_t li) {
+            const DevTensor* tp = tensors + ti;
+            const HyperDev& h = SCHED ? sched_h[tp->hyper] : hp.h[tp->hyper];
+            if (DT == 1 || (DT == 0 && tp->dtype == QF_BF16))
+                main_strip<__nv_bfloat16, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
+            else if (DT == 3 || (DT == 0 && tp->dtype == QF_F16))
+                main_strip<__half, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
+            else
+                main_strip<float, PUSH>(tp, li, h, s, words, words + kStripWords, status, push);
+        });
+    }
+    if ((MAP == kMapFlat || MAP == kMapAll) && map == kMapFlat) {
+        for_items<true>(w, kMapFlat, part, [&](int ti, int64_t li) {
+            const DevTensor* tp = tensors + ti;
+            const HyperDev& h = SCHED ? sched_h[tp->hyper] : hp.h[tp->hyper];
+            if (DT == 1 || (DT == 0 && tp->dtype == QF_BF16))
                 main_flat_dispatch<__nv_bfloat16>(tp, li, h, s, status, push);
-            else if (tp->dtype == QF_F16)
+            else if (DT == 3 || (DT == 0 && tp->dtype == QF_F16))
                 main_flat_dispatch<__half>(tp, li, h, s, status, push);
             else
                 main_flat_dispatch<float>(tp, li, h, s, status, push);
-        }
+        });
     }
-    for (int i = blockIdx.x; i < n_roll; i += gridDim.x) roll_item(tensors, roll_base, n, i, kRollCommit);
+    for (int i = blockIdx.x; i < n_roll; i += gridDim.x) roll_item(tensors, roll_base, w.n, i, kRollCommit);
 }
 
 // One tensor passed by value (the single-tensor entry points that mirror the reference's per-tensor
