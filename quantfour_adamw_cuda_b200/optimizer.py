@@ -70,7 +70,12 @@ class _DevicePlan:
         self.descs = None
         self.workspace: Optional[torch.Tensor] = None
         self.keepalive: list = []
+        self.workspace_ptr = self.workspace_bytes = 0
         self.nd: list = []      # (parameter, second-moment overhead) of the tensors of three and more dimensions with per-axis maxima
+
+    def take_workspace(self, need: int, dev: torch.device) -> None:
+        self.workspace = torch.zeros(need, dtype=torch.uint8, device=dev)
+        self.workspace_ptr, self.workspace_bytes = self.workspace.data_ptr(), self.workspace.numel()
 
 
 class FourBitAdamW(torch.optim.Optimizer):
@@ -300,7 +305,6 @@ class FourBitAdamW(torch.optim.Optimizer):
             lead = mx if lead is None else torch.minimum(lead, mx)
         rm.copy_(lead)
 
-    @torch.no_grad()
     def step(self, closure=None, *, grad_scale: Optional[float] = None):
         """Perform a single optimization step (fused_quantfour.py:131-138); returns the closure's loss.
 
@@ -314,12 +318,17 @@ class FourBitAdamW(torch.optim.Optimizer):
                 loss = closure()
         self._grad_scale = 1.0 if grad_scale is None else float(grad_scale)
 
-        if self.capturable:
-            self._step_capturable()
+        if not self.capturable and self._fast is not None and self._step_fast():
             return loss
-        if self._fast is not None and self._step_fast():
-            return loss
+        with torch.no_grad():
+            if self.capturable:
+                self._step_capturable()
+            else:
+                self._step_general()
+        return loss
 
+    def _step_general(self) -> None:
+        """A step from the parameter list alone: state, descriptors and hyper-parameters built anew."""
         hypers: List[_lib.QfHyper] = []
         hyper_index: Dict[tuple, int] = {}
         work: Dict[torch.device, List[tuple]] = {}
@@ -369,7 +378,6 @@ class FourBitAdamW(torch.optim.Optimizer):
         self._fast = None
         if cacheable and len(work) == 1 and len(hypers) <= _lib.QF_MAX_HYPERS:
             self._remember(next(iter(work.items())), hyper_index)
-        return loss
 
     # ---- steady state: same tensors, same gradient buffers as the step before ---------------------------
 
@@ -396,17 +404,23 @@ class FourBitAdamW(torch.optim.Optimizer):
         self._fast = {
             "dev": dev, "plan": self._plans[(dev.index, 0)], "checks": [(p, p.data_ptr(), g.data_ptr()) for p, g, _, _ in entries],
             "absent": [p for g in self.param_groups for p in g["params"] if id(p) not in seen],
-            "steps_vec": steps_vec, "classes": classes, "stream": torch.cuda.current_stream(dev).cuda_stream,
-            "n_params": sum(len(g["params"]) for g in self.param_groups),
+            "steps_vec": steps_vec, "classes": classes, "stream": torch._C._cuda_getCurrentRawStream(dev.index),
+            "n_params": sum(len(g["params"]) for g in self.param_groups), "harr": (_lib.QfHyper * len(classes))(),
         }
 
     def _step_fast(self) -> bool:
+        # All a small step costs on the host beside its launches, so it looks at each parameter once and calls torch for
+        # the step counters only.
         f = self._fast
-        if f["n_params"] != sum(len(g["params"]) for g in self.param_groups):
+        groups = self.param_groups
+        n_params = 0
+        for g in groups:
+            n_params += len(g["params"])
+        if f["n_params"] != n_params:
             return False
         plan = f["plan"]
         checks = f["checks"]
-        moved = []
+        moved = None
         for i, (p, pptr, gptr) in enumerate(checks):
             g = p.grad
             if g is None or p.data_ptr() != pptr:
@@ -414,48 +428,51 @@ class FourBitAdamW(torch.optim.Optimizer):
             if g.data_ptr() != gptr:     # a new gradient buffer: only its address in the descriptor changes
                 if not g.is_contiguous() or g.dtype != p.dtype or g.numel() != p.numel() or g.is_sparse:
                     return False
+                moved = moved or []
                 moved.append((i, g))
         for p in f["absent"]:
             if p.grad is not None:
                 return False
-        for c in f["classes"]:
-            if float(c[2]) != c[1]:      # somebody rewrote a step counter: rebuild the classes
+        classes = f["classes"]
+        for c in classes:
+            if c[2].item() != c[1]:      # somebody rewrote a step counter: rebuild the classes
                 return False
-        for i, g in moved:
-            plan.descs[i].g = g.data_ptr()
-            plan.keepalive[i] = g
-            checks[i] = (checks[i][0], checks[i][1], g.data_ptr())
         if moved:
+            for i, g in moved:
+                plan.descs[i].g = g.data_ptr()
+                plan.keepalive[i] = g
+                checks[i] = (checks[i][0], checks[i][1], g.data_ptr())
             plan.signature = None     # the slow path must not trust its cached signature any more
         f["steps_vec"].add_(1.0)
-        hypers = []
-        for c in f["classes"]:
+        harr = f["harr"]
+        for k, c in enumerate(classes):
             c[1] += 1.0
-            group = self.param_groups[c[0]]
+            group = groups[c[0]]
             beta1, beta2 = group["betas"]
-            hypers.append(make_hyper(group["lr"], beta1, beta2, group["eps"], group["weight_decay"], c[1], self._grad_scale))
-        dev = f["dev"]
-        harr = (_lib.QfHyper * len(hypers))(*hypers)
+            harr[k] = make_hyper(group["lr"], beta1, beta2, group["eps"], group["weight_decay"], c[1], self._grad_scale)
         # the table of these descriptors is in the workspace since the last call, unless a gradient moved or the step
         # now runs on another stream than the one the table was copied on
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        self._run(plan, harr, len(hypers), dev, table_in_place=not moved and f.get("stream") == stream)
+        dev = f["dev"]
+        stream = torch._C._cuda_getCurrentRawStream(dev.index)
+        self._run(plan, harr, len(classes), dev, not moved and f["stream"] == stream, stream)
         f["stream"] = stream
         return True
 
-    def _run(self, plan, harr, n_hypers: int, dev: torch.device, table_in_place: bool) -> None:
+    def _run(self, plan, harr, n_hypers: int, dev: torch.device, table_in_place: bool, stream: int) -> None:
         """Both halves of the step on `plan`; `table_in_place`: the workspace holds the table of plan.descs already."""
         flags = (_lib.QF_RUN_RELAXED_UPDATE if self.relaxed_update else 0) | (_lib.QF_RUN_TABLE_IN_PLACE if table_in_place else 0)
-        L = _lib.lib()
-        args = (plan.descs, len(plan.descs), harr, n_hypers, plan.workspace.data_ptr(), plan.workspace.numel(), dev.index,
-                C.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+        run = _lib.lib().qf_step_run
+        args = (plan.descs, len(plan.descs), harr, n_hypers, plan.workspace_ptr, plan.workspace_bytes, dev.index, stream)
         if not plan.nd:
-            _lib.check(L.qf_step_run(*args, _lib.QF_RUN_PRE | _lib.QF_RUN_MAIN | flags, None, 0), "qf_step_run")
+            rc = run(*args, _lib.QF_RUN_PRE | _lib.QF_RUN_MAIN | flags, None, 0)
+            if rc:
+                _lib.check(rc, "qf_step_run")
             return
-        _lib.check(L.qf_step_run(*args, _lib.QF_RUN_PRE | flags, None, 0), "qf_step_run")
-        for p, vo in plan.nd:
-            self._fold_new_maxima(p, vo)
-        _lib.check(L.qf_step_run(*args, _lib.QF_RUN_MAIN | _lib.QF_RUN_TABLE_IN_PLACE | flags, None, 0), "qf_step_run")
+        _lib.check(run(*args, _lib.QF_RUN_PRE | flags, None, 0), "qf_step_run")
+        with torch.no_grad():
+            for p, vo in plan.nd:
+                self._fold_new_maxima(p, vo)
+        _lib.check(run(*args, _lib.QF_RUN_MAIN | _lib.QF_RUN_TABLE_IN_PLACE | flags, None, 0), "qf_step_run")
 
     def _launch(self, dev: torch.device, chunk: int, entries: List[tuple], hypers: List[_lib.QfHyper], hyper_base: int) -> None:
         L = _lib.lib()
@@ -469,13 +486,13 @@ class FourBitAdamW(torch.optim.Optimizer):
                 self._fill_desc(d, p, g, st, hi - hyper_base)
             need = L.qf_workspace_bytes(n)
             if plan.workspace is None or plan.workspace.numel() < need or plan.workspace.device != dev:
-                plan.workspace = torch.zeros(need, dtype=torch.uint8, device=dev)
+                plan.take_workspace(need, dev)
             plan.descs, plan.signature = descs, signature
             plan.keepalive = [g for _, g, _, _ in entries]
             plan.nd = [(p, st["variance_qstate"]["overhead"]) for p, _, st, _ in entries
                        if st["momentum_qstate"]["enable"] and len(st["variance_qstate"]["overhead"].get("max_dims") or ()) > 2]
         harr = (_lib.QfHyper * len(hypers))(*hypers)
-        self._run(plan, harr, len(hypers), dev, table_in_place=False)
+        self._run(plan, harr, len(hypers), dev, False, torch._C._cuda_getCurrentRawStream(dev.index))
 
     def _read_status(self) -> None:
         """Synchronise, fold the status word of every workspace into `_status_bits` and clear the words."""
@@ -619,7 +636,7 @@ class FourBitAdamW(torch.optim.Optimizer):
             self._fill_desc(d, p, g, st, ci)
         need = L.qf_workspace_bytes(n)
         if plan.workspace is None or plan.workspace.numel() < need or plan.workspace.device != dev:
-            plan.workspace = torch.zeros(need, dtype=torch.uint8, device=dev)
+            plan.take_workspace(need, dev)
         plan.descs, plan.signature, plan.keepalive = descs, None, [g for _, g, _, _ in entries]
         stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         _lib.check(L.qf_step_prepare(descs, n, len(classes), plan.workspace.data_ptr(), plan.workspace.numel(), dev.index, stream),
