@@ -95,7 +95,8 @@ struct HyperPack {
 };
 
 // The scalars as the kernels take them.  The packed sequences of the fast path need: finite scalars, an
-// eps that absorbs the square root of a denormal second moment (>= 2^-40), a bias correction whose
+// eps that absorbs the square root of a denormal second moment (>= 2^-40), a beta2 that keeps a second moment of normal
+// size normal, a bias correction whose
 // reciprocal is well defined, and a non-degenerate step size; anything else runs the exact path.
 // Host and device give the same result: the one division is an IEEE double division on both.
 __host__ __device__ inline HyperDev widen_hyper(const QfHyper& h) {
@@ -108,7 +109,7 @@ __host__ __device__ inline HyperDev widen_hyper(const QfHyper& h) {
     bool ok = true;
     for (float x : all) ok = ok && fabsf(x) <= 3.4028234663852886e38f;  // finite: false for NaN and infinities
     ok = ok && h.eps >= 0x1p-40f && h.eps <= 0x1p40f && h.bc2s >= 0x1p-30f && h.bc2s <= 2.0f;
-    ok = ok && fabsf(h.neg_step) <= 0x1p40f && fabsf(h.decay) <= 0x1p40f && h.beta2 >= 0.0f && h.w2 >= 0.0f;
+    ok = ok && fabsf(h.neg_step) <= 0x1p40f && fabsf(h.decay) <= 0x1p40f && h.beta2 >= 0x1p-6f && h.w2 >= 0.0f;
     d.fast = ok ? 1 : 0;
     return d;
 }
@@ -263,6 +264,7 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, int j) {
     return j == 0 ? (w & 0xffu) : j == 3 ? (w >> 24) : prmt(w, 0u, 0x4440u + j);
 }
+__device__ __forceinline__ uint32_t byte_of_any(uint32_t w, int j) { return (w >> (8 * j)) & 0xffu; }   // j not a constant
 // The two bf16 values of a word as floats (low half first): byte permutes, which keep the shift off the
 // multiply-add pipe where the compiler would otherwise place it.
 __device__ __forceinline__ f2 widen_bf16x2(uint32_t w) {
@@ -612,17 +614,16 @@ __device__ __noinline__ float main_panel_row_exact(const DevTensor* tp, int64_t 
 // ever reads what it copied itself, so the slots need no barrier: cp.async.wait_group orders a lane's
 // copies with its own reads.  One row ahead per warp is enough at two CTAs per SM (a third slot measured
 // slower, and so did bulk copies with an mbarrier per slot: four 128..512-byte requests per row and warp are too
-// small for the copy engine).  The per-lane column maxima (old, new, reciprocal of new) sit in shared memory as
-// well and are fetched pair by pair: registers are the scarce resource of this kernel (keeping them in registers
+// small for the copy engine).  The per-lane column maxima (old, new) sit in shared memory as well and are fetched pair by pair: registers are the scarce resource of this kernel (keeping them in registers
 // measured 8 % slower at 128 registers per thread).
 constexpr int kStages = 2;                             // this row and the next one
 constexpr int kRowBytesBf16 = 32 * (2 * 16 + 8);       // staged bytes of one row of a panel, bf16 parameters
 constexpr int kRowBytesF32 = 32 * (2 * 2 * 16 + 8);    // the same for fp32 parameters
-constexpr int kColBytes = 3 * 4 * 32 * 8;              // per warp: old / new / reciprocal column maxima of its 256 columns
+constexpr int kColBytes = 2 * 4 * 32 * 8;              // per warp: old and new column maxima of its 256 columns
 // Dynamic shared memory of the panel kernel: per warp the two slots plus the column block.  The host sizes the
 // slots for fp32 rows only when the launch holds an fp32 panel tensor: less shared memory leaves more L1 to the
 // CTA, which the measurements reward.
-constexpr int kRowBufBytes = 2 * kMainRowsPerItem * 16;  // per warp: the scalars of every row of its item, once per 128-block
+constexpr int kRowBufBytes = kMainRowsPerItem * 16;    // per warp: the scalars of every row of its item
 constexpr int main_dyn_smem(bool any_f32) {
     return kWarpsPerCta * (kStages * (any_f32 ? kRowBytesF32 : kRowBytesBf16) + kColBytes + kRowBufBytes);
 }
@@ -650,6 +651,26 @@ __device__ __forceinline__ void adamw_pair_panel(f2& p, f2 g, f2& m, f2& v, cons
     const f2 den = add2(BC1 ? s : div2_prepared_n<P1>(s, h.rb, h.nb), h.eps);
     const f2 a = mul2(h.nstep, m);
     p = add2(p1, P1 ? div2_1(a, den) : div2(a, den));
+}
+
+// The update of two 16-bit parameters without the corrections of the exact sequences, but with a proof.  The quotient
+// q = nstep * m / den is taken from the approximations of the square root, of 1 / bc2s and of the reciprocal.  Against the
+// exactly rounded sequence of operations its relative error is below 2^-22.9 (rsqrt) + 2^-23 (rcp) + 8 * 2^-24 (the
+// roundings of either sequence) < 2^-20.3.  The exact sum is RN(p1 + q*) with q* between q (1 - 2^-20) and q (1 + 2^-20), so
+// by monotonicity of the roundings the new parameter lies between the two sums lo and hi rounded to 16 bits: where these
+// agree (all but about 2^-11 |q / p| of the elements) they are the exact result.  Six packed operations instead of
+// thirteen (bf16) or eighteen (fp16); `differ` collects the bits in which lo and hi disagree.
+template <typename T, bool BC1>
+__device__ __forceinline__ uint32_t adamw_pair_bracket(f2 p, f2 g, f2& m, f2& v, const Hyper2& h, uint32_t& differ) {
+    const f2 p1 = fma2(p, h.decay, bc2(0.0f));
+    m = fma2(h.w1, add2(g, neg2(m)), m);
+    v = fma2(mul2(h.w2, g), g, mul2(h.beta2, v));
+    const f2 y = mk2(rsqrt_approx(v.x), rsqrt_approx(v.y));
+    const f2 den = BC1 ? fma2(v, y, h.eps) : fma2(mul2(v, y), h.rb, h.eps);
+    const f2 q = mul2(mul2(h.nstep, m), mk2(rcp_approx(den.x), rcp_approx(den.y)));
+    const uint32_t lo = pack16<T>(fma2(q, bc2(1.0f - 0x1p-20f), p1)), hi = pack16<T>(fma2(q, bc2(1.0f + 0x1p-20f), p1));
+    differ |= lo ^ hi;
+    return lo;
 }
 
 // Second pass over one item of a rank-1 panel: 64 rows of 256 columns.
@@ -695,58 +716,52 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
         cp_async4(lane_codes + slot_off + 128, vc + (e >> 1));
     };
 
-    float4* colbuf = reinterpret_cast<float4*>(stage + ring_bytes) + lane;  // [old | -new | 1/new][half][lane]
+    float4* colbuf = reinterpret_cast<float4*>(stage + ring_bytes) + lane;  // [old | -new][half][lane]
     bool ok = hd.fast;
     {
-        float col_old[8], col_new[8], rcol[8];
+        float col_old[8], col_new[8];
         load8f(t.vcol_old, j0, col_old);
         load8f(t.vcol_new, j0, col_new);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            rcol[k] = col_new[k] == 0.0f ? 0.0f : __frcp_rn(col_new[k]);
-            ok &= scale_safe(col_new[k]) && scale_safe(col_old[k]) && col_old[k] > 0.0f;
-        }
+        for (int k = 0; k < 8; ++k) ok &= scale_safe(col_new[k]) && scale_safe(col_old[k]) && col_old[k] > 0.0f;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             colbuf[(0 * 2 + j) * 32] = make_float4(col_old[4 * j], col_old[4 * j + 1], col_old[4 * j + 2], col_old[4 * j + 3]);
             colbuf[(1 * 2 + j) * 32] = make_float4(-col_new[4 * j], -col_new[4 * j + 1], -col_new[4 * j + 2], -col_new[4 * j + 3]);
-            colbuf[(2 * 2 + j) * 32] = make_float4(rcol[4 * j], rcol[4 * j + 1], rcol[4 * j + 2], rcol[4 * j + 3]);
         }
     }
     const bool col_fast = __all_sync(kFull, ok);
     const Hyper2 h2 = widen(hd);
 
-    // The scalars of the item's rows: (old maximum, -new maximum, 1 / new maximum, old block scale), one entry per row
-    // and 128-block, fetched a row per lane and read back by the whole warp with one broadcast load per row (four
-    // global loads with their addresses per row before).  The reciprocal is NaN where the row cannot take the packed
-    // arithmetic: a maximum outside the range of the division sequences or an old maximum of zero.  The row's new
-    // block scale replaces the old one and goes out with the others at the end of the item.
+    // The scalars of the item's rows: (old maximum, -new maximum, old scales of the row's two 128-blocks), fetched a row per
+    // lane and read back by the whole warp with one broadcast load per row (four global loads with their addresses per
+    // row before).  The old maximum is NaN where the row cannot take the packed arithmetic: a maximum outside the range
+    // of the division sequences.  The row's new block scales replace the old ones and go out together at the end of the item.
     float4* const rowbuf = reinterpret_cast<float4*>(stage + ring_bytes + kColBytes);
     const uint32_t block0 = (static_cast<uint32_t>(r0) * cols + panel * kPanelCols) >> 7, row_blocks = cols >> 7;
     for (int k = lane; k < r1 - r0; k += 32) {
         const float old = __ldg(t.vrow_old + r0 + k), nw = __ldg(t.vrow_new + r0 + k);
         const float* ms = t.ms + block0 + static_cast<uint32_t>(k) * row_blocks;
-        const float rr = nw == 0.0f ? 0.0f : __frcp_rn(nw);
-        const bool fit = scale_safe(nw) && scale_safe(old) && old > 0.0f;
-        float4 e4 = make_float4(old, -nw, fit ? rr : __uint_as_float(0x7fc00000u), ms[0]);
-        rowbuf[k] = e4;
-        e4.w = ms[1];
-        rowbuf[kMainRowsPerItem + k] = e4;
+        rowbuf[k] = make_float4(scale_safe(nw) && scale_safe(old) ? old : __uint_as_float(0x7fc00000u), -nw, ms[0], ms[1]);
     }
     __syncwarp();
-    float4* const my_rows = rowbuf + (lane >> 4) * kMainRowsPerItem;   // the entries of this lane's 128-block
+    const bool upper = lane & 16;   // this lane's values lie in the second 128-block
+    auto keep_scale = [&](int k_row, float ms_new) {
+        if ((lane & 15) == 0) reinterpret_cast<float*>(rowbuf + k_row)[upper ? 3 : 2] = ms_new;
+    };
 
+    auto store_words = [&](uint32_t e, const uint32_t (&w)[4]) {   // eight 16-bit parameters
+        const uint4 out = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(t.p + static_cast<size_t>(e) * 2) = out;
+        if (PUSH) {
+            const int n = push->n;
+            for (int k = 0; k < n; ++k) *reinterpret_cast<uint4*>(t.p + push->delta[k] + static_cast<size_t>(e) * 2) = out;
+        }
+    };
     auto store_p = [&](uint32_t e, const f2 (&pp)[4]) {
         if (H16) {
-            uint32_t w[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = pack16<T>(pp[j]);
-            const uint4 out = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4*>(t.p + static_cast<size_t>(e) * 2) = out;
-            if (PUSH) {
-                const int n = push->n;
-                for (int k = 0; k < n; ++k) *reinterpret_cast<uint4*>(t.p + push->delta[k] + static_cast<size_t>(e) * 2) = out;
-            }
+            const uint32_t w[4] = {pack16<T>(pp[0]), pack16<T>(pp[1]), pack16<T>(pp[2]), pack16<T>(pp[3])};
+            store_words(e, w);
         } else {
             const float4 o0 = make_float4(pp[0].x, pp[0].y, pp[1].x, pp[1].y), o1 = make_float4(pp[2].x, pp[2].y, pp[3].x, pp[3].y);
             float4* dst = reinterpret_cast<float4*>(t.p + static_cast<size_t>(e) * 4);
@@ -766,7 +781,8 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
     // One row out of the staging slot at `slot_off`.  False: the row cannot take the packed arithmetic; nothing of
     // it has been stored.
     auto row = [&](int k_row, uint32_t e, int slot_off) -> bool {
-        const float4 sc = my_rows[k_row];
+        const float4 sc = rowbuf[k_row];
+        const float ms = upper ? sc.w : sc.z;
         // the staged row as it was copied: four words of two bf16 values, or eight floats, per array
         uint32_t pw[NV * 4], gw[NV * 4];
 #pragma unroll
@@ -777,16 +793,17 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
             gw[4 * v] = b.x; gw[4 * v + 1] = b.y; gw[4 * v + 2] = b.z; gw[4 * v + 3] = b.w;
         }
         f2 pp[4];
+        uint32_t pout[4], differ = 0;   // 16-bit parameters: the new words
         const uint32_t wm = *reinterpret_cast<const uint32_t*>(lane_codes + slot_off);
         const uint32_t wv = *reinterpret_cast<const uint32_t*>(lane_codes + slot_off + 128);
-        const f2 ms_old = bc2(sc.w);
-        const float row_old = sc.x, nrow = sc.y, rrow = sc.z;
+        const f2 ms_old = bc2(ms);
+        const float row_old = sc.x, nrow = sc.y;
         f2 m[4];
         if (__any_sync(kFull, row_old == 0.0f)) {
             // A row without second moment (a token that has not occurred, the padding of a vocabulary): where its first
             // moment and its gradient are zero as well, the moments stay zero -- codes of x = 0, scale 0 -- and the
             // parameter only decays (the quotient of the update is a zero of the first moment's sign).
-            uint32_t any = __float_as_uint(sc.w);
+            uint32_t any = __float_as_uint(ms);
 #pragma unroll
             for (int j = 0; j < NV * 4; ++j) any |= gw[j] & (H16 ? 0x7fff7fffu : 0x7fffffffu);
             if (__any_sync(kFull, any != 0)) return false;
@@ -808,21 +825,26 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
             pp[j] = H16 ? widen16<T>(pw[j]) : mk2(__uint_as_float(pw[(2 * j) % (NV * 4)]), __uint_as_float(pw[(2 * j + 1) % (NV * 4)]));
             const f2 gg = H16 ? widen16<T>(gw[j]) : mk2(__uint_as_float(gw[(2 * j) % (NV * 4)]), __uint_as_float(gw[(2 * j + 1) % (NV * 4)]));
             m[j] = mul2(pair_entry(s.qm2, wm, j), ms_old);
-            const float4 a = colbuf[(0 * 2 + (j >> 1)) * 32], b = colbuf[(1 * 2 + (j >> 1)) * 32], c = colbuf[(2 * 2 + (j >> 1)) * 32];
+            const float4 a = colbuf[(0 * 2 + (j >> 1)) * 32], b = colbuf[(1 * 2 + (j >> 1)) * 32];
             const f2 co = (j & 1) ? mk2(a.z, a.w) : mk2(a.x, a.y);
             const f2 ncn = (j & 1) ? mk2(b.z, b.w) : mk2(b.x, b.y);
-            const f2 rcn = (j & 1) ? mk2(c.z, c.w) : mk2(c.x, c.y);
             f2 v = mul2(pair_entry(s.qv2, wv, j), mk2(fminf(row_old, co.x), fminf(row_old, co.y)));
-            adamw_pair_panel<BF16, BC1, RELAXED>(pp[j], gg, m[j], v, h2);
-            // requantize v: scale = min(row', col') -> -scale = max(-row', -col'), 1/scale = max(1/row', 1/col')
+            if (H16 && !RELAXED)
+                pout[j] = adamw_pair_bracket<T, BC1>(pp[j], gg, m[j], v, h2, differ);
+            else
+                adamw_pair_panel<BF16, BC1, RELAXED>(pp[j], gg, m[j], v, h2);
+            // requantize v: scale = min(row', col') -> -scale = max(-row', -col').  Its reciprocal from the approximation unit:
+            // keeping those of the row and column maxima and taking their maximum is two instructions as well, and eight
+            // more shared-memory wavefronts per row (second pass over 645 M elements 1350 -> 1321 us without them).  A zero
+            // scale gives NaN, which the conversion turns into code 0 as the rule for all-zero groups has it.
             const f2 nsv = mk2(fmaxf(nrow, ncn.x), fmaxf(nrow, ncn.y));
-            const f2 rv = mk2(fmaxf(rrow, rcn.x), fmaxf(rrow, rcn.y));
+            const f2 rv = mk2(rcp_approx(-nsv.x), rcp_approx(-nsv.y));
             const f2 y = fma2(div2_prepared1(v, rv, nsv), bc2(16.0f), bc2(-1.5f));
             cv[2 * j] = ceil_s32(y.x);       // x <= 1 here (the scale is a maximum over values that include v): at most 15
             cv[2 * j + 1] = ceil_s32(y.y);
         }
         const float ms_new = absmax_pairs_to_block(m);
-        const bool row_ok = rrow == rrow && sc.w < __builtin_huge_valf() && scale_safe(ms_new);
+        const bool row_ok = row_old == row_old && ms < __builtin_huge_valf() && scale_safe(ms_new);
         if (!__all_sync(kFull, row_ok)) return false;     // the vote also tells the compiler that the branch is uniform
         uint32_t wmq;
         {
@@ -838,10 +860,30 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
             wmq = pack_u4(c[1], c[0], pack_u4(c[3], c[2], pack_u4(c[5], c[4], pack_u4(c[7], c[6], 0u))));
         }
         const uint32_t wq = pack_u4(cv[1], cv[0], pack_u4(cv[3], cv[2], pack_u4(cv[5], cv[4], pack_u4(cv[7], cv[6], 0u))));
-        store_p(e, pp);
+        if (H16 && !RELAXED) {
+            if (__any_sync(kFull, differ != 0)) {
+                // some parameter next to a rounding boundary: the exact sequence for the row, from the staged inputs
+#pragma unroll 1
+                for (int j = 0; j < 4; ++j) {
+                    f2 p = widen16<T>(*reinterpret_cast<const uint32_t*>(lane_vec + slot_off + 4 * j));
+                    const f2 gg = widen16<T>(*reinterpret_cast<const uint32_t*>(lane_vec + slot_off + kArr + 4 * j));
+                    const float2 co = reinterpret_cast<const float2*>(colbuf + (j >> 1) * 32)[j & 1];
+                    f2 m1 = mul2(s.qm2.v[byte_of_any(*reinterpret_cast<const uint32_t*>(lane_codes + slot_off), j)], ms_old);
+                    f2 v1 = mul2(s.qv2.v[byte_of_any(*reinterpret_cast<const uint32_t*>(lane_codes + slot_off + 128), j)],
+                                 mk2(fminf(row_old, co.x), fminf(row_old, co.y)));
+                    adamw_pair<true, BC1>(p, gg, m1, v1, h2);
+                    const uint32_t w = pack16<T>(p);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) pout[i] = i == j ? w : pout[i];
+                }
+            }
+            store_words(e, pout);
+        } else {
+            store_p(e, pp);
+        }
         *reinterpret_cast<uint32_t*>(vc + (e >> 1)) = wq;
         *reinterpret_cast<uint32_t*>(mc + (e >> 1)) = wmq;
-        if ((lane & 15) == 0) my_rows[k_row].w = ms_new;
+        keep_scale(k_row, ms_new);
         return true;
     };
 
@@ -873,15 +915,15 @@ __device__ __forceinline__ void main_panel(const DevTensor* tp, int64_t li, cons
         }
         if (r < r1) {  // cold: this row exactly, from its unmodified inputs
             const float ms_new = main_panel_row_exact<T>(tp, static_cast<uint32_t>(r) * cols + j0, r, j0, hd, s, status, PUSH ? push : nullptr);
-            if ((lane & 15) == 0) my_rows[r - r0].w = ms_new;
+            keep_scale(r - r0, ms_new);
             ++r;
         }
     }
     __syncwarp();
     for (int k = lane; k < r1 - r0; k += 32) {
         float* ms = t.ms + block0 + static_cast<uint32_t>(k) * row_blocks;
-        ms[0] = rowbuf[k].w;
-        ms[1] = rowbuf[kMainRowsPerItem + k].w;
+        ms[0] = rowbuf[k].z;
+        ms[1] = rowbuf[k].w;
     }
     __syncwarp();   // the next item of this warp fills the buffer again
 }

@@ -90,3 +90,15 @@ def test_quantize_and_dequantize_blocks_of_short_items(n, mid, qmap, quantize, d
     want_codes, want_scales = TO.quantize_block(x, getattr(TO, mid))
     assert torch.equal(codes.cpu().view(torch.uint8), want_codes) and torch.equal(scales.cpu(), want_scales)
     assert torch.equal(getattr(F, dequantize)(codes, scales, n).cpu(), TO.dequantize_block(want_codes, want_scales, n, getattr(TO, qmap)))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("lr", [3e-7, 1e-2, 1.0])
+def test_parameters_next_to_rounding_boundaries(dtype, lr, monkeypatch):
+    """Updates much smaller than, comparable to and much larger than the parameter: the 16-bit rounding of the new parameter is
+    decided by the update's last places for anything from no element of a row to several in every row."""
+    import sys
+    me = sys.modules[__name__]
+    monkeypatch.setattr(me, "HP", dict(HP, lr=lr))
+    monkeypatch.setattr(me, "ARGS", (lr, *HP["betas"], HP["eps"], HP["weight_decay"]))
+    run([((512, 1024), dtype), ((700, 555), dtype), ((300_000,), dtype)], steps=5)
