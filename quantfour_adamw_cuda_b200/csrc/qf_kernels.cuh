@@ -1116,6 +1116,36 @@ __device__ __forceinline__ void main_flat_run_fp32(const DevTensor& t, int64_t w
     Elem<float>::store8(t.v, e, v);
 }
 
+// A lane's eight new parameters: 16-bit ones come packed, fp32 ones as they are.
+template <typename T>
+__device__ __forceinline__ void store_params(char* base, int64_t e, const float (&p)[8], const uint32_t (&packed)[4], const PushPack* push) {
+    if (sizeof(T) != 2) {
+        Elem<T>::store8(base, e, p);
+        if (push) push_store8<T>(base, e, p, push);
+        return;
+    }
+    const uint4 out = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    *reinterpret_cast<uint4*>(base + e * 2) = out;
+    for (int k = 0, n = push ? push->n : 0; k < n; ++k) *reinterpret_cast<uint4*>(base + push->delta[k] + e * 2) = out;
+}
+// The exact sequence for a lane's eight 16-bit parameters (see adamw_pair_bracket), from their unmodified inputs in memory:
+// rarely taken, so it keeps nothing of them in registers.  scale(j): the second-moment scales of pair j.
+template <typename T, typename Scale>
+__device__ __forceinline__ void exact_params(const DevTensor& t, int64_t e, const Hyper2& h2, const Smem& s, f2 ms_old, Scale scale,
+                                             uint32_t (&packed)[4]) {
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+        f2 p = widen16<T>(*reinterpret_cast<const uint32_t*>(t.p + (e + 2 * j) * 2));
+        const f2 g = widen16<T>(*reinterpret_cast<const uint32_t*>(t.g + (e + 2 * j) * 2));
+        f2 m = mul2(s.qm2.v[*reinterpret_cast<const uint8_t*>(t.m + (e >> 1) + j)], ms_old);
+        f2 v = mul2(s.qv2.v[*reinterpret_cast<const uint8_t*>(t.v + (e >> 1) + j)], scale(j));
+        adamw_pair<true>(p, g, m, v, h2);
+        const uint32_t w = pack16<T>(p);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) packed[i] = i == j ? w : packed[i];
+    }
+}
+
 // A lane's inputs of one full run of a block-128 tensor, as loaded.
 template <typename T>
 struct BlockRun {
@@ -1144,12 +1174,16 @@ __device__ __forceinline__ bool main_flat_run_block(const DevTensor& t, int64_t 
     const f2 ms_old = bc2(in.ms), vs_old = bc2(in.vs);
     f2 m[4], v[4];
     float low = __builtin_huge_valf();
+    uint32_t pout[4], differ = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         f2 pp = mk2(p[2 * j], p[2 * j + 1]);
         m[j] = mul2(pair_entry(s.qm2, in.wm, j), ms_old);
         v[j] = mul2(pair_entry(s.qv2, in.wv, j), vs_old);
-        adamw_pair<true>(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v[j], h2);
+        if (sizeof(T) == 2)
+            pout[j] = adamw_pair_bracket<T, false>(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v[j], h2, differ);
+        else
+            adamw_pair<true>(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v[j], h2);
         low = fminf(low, fminf(v[j].x, v[j].y));
         p[2 * j] = pp.x;
         p[2 * j + 1] = pp.y;
@@ -1157,8 +1191,9 @@ __device__ __forceinline__ bool main_flat_run_block(const DevTensor& t, int64_t 
     const float ms_new = absmax_pairs_to_block_nan(m);   // no first pass vouches for these values: a NaN must survive
     const float vs_new = absmax_pairs_to_block_nan(v);
     if (!__all_sync(kFull, low >= 0x1p-96f && scale_safe(ms_new) && scale_safe(vs_new))) return false;
-    Elem<T>::store8(t.p, e, p);
-    if (push) push_store8<T>(t.p, e, p, push);
+    if (sizeof(T) == 2 && __any_sync(kFull, differ != 0))
+        exact_params<T>(t, e, h2, s, ms_old, [&](int) { return vs_old; }, pout);
+    store_params<T>(t.p, e, p, pout, push);
     *reinterpret_cast<uint32_t*>(t.m + (e >> 1)) = quantize_m8_safe(m, ms_new, s);
     const f2 r2 = bc2(__frcp_rn(vs_new)), ns2 = bc2(-vs_new);
     int c[8];
@@ -1369,8 +1404,7 @@ __device__ __forceinline__ void pre_strip(const DevTensor& t, int64_t li, const 
     __syncthreads();   // the next item fills the arrays again
 }
 
-// Second pass over a strip.  A full run takes the packed arithmetic -- with correctly rounded divisions for every dtype,
-// as the exact path has them -- where its scalars allow it (old and new maxima of its rows and of the strip's columns in
+// Second pass over a strip.  A full run takes the packed arithmetic where its scalars allow it (old and new maxima of its rows and of the strip's columns in
 // [2^-80, 2^100], the old first-moment scale finite, the new one zero or in range); any other run goes through
 // main_flat_run_exact.  Nothing of a run is stored before that is known.
 __device__ __forceinline__ bool strip_scale_ok(float x) { return x >= 0x1p-80f && x <= 0x1p100f; }
@@ -1415,6 +1449,7 @@ __device__ __forceinline__ void main_strip(const DevTensor* tp, int64_t li, cons
             g_raw.widen(g);
             f2 m[4];
             int cv[8];
+            uint32_t pout[4], differ = 0;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int w0 = strip_word(first, 2 * j), w1 = strip_word(first, 2 * j + 1);
@@ -1424,7 +1459,10 @@ __device__ __forceinline__ void main_strip(const DevTensor* tp, int64_t li, cons
                 f2 pp = mk2(p[2 * j], p[2 * j + 1]);
                 f2 v = mul2(pair_entry(s.qv2, wv, j), so);
                 m[j] = mul2(pair_entry(s.qm2, wm, j), bc2(ms));
-                adamw_pair<true>(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v, h2);
+                if (sizeof(T) == 2)
+                    pout[j] = adamw_pair_bracket<T, false>(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v, h2, differ);
+                else
+                    adamw_pair<true>(pp, mk2(g[2 * j], g[2 * j + 1]), m[j], v, h2);
                 p[2 * j] = pp.x;
                 p[2 * j + 1] = pp.y;
                 const f2 y = fma2(div2(v, sn), bc2(16.0f), bc2(-1.5f));
@@ -1433,8 +1471,12 @@ __device__ __forceinline__ void main_strip(const DevTensor* tp, int64_t li, cons
             }
             const float ms_new = absmax_pairs_to_block_nan(m);
             if (__all_sync(kFull, ok && scale_safe(ms_new))) {
-                Elem<T>::store8(t.p, e, p);
-                if (PUSH) push_store8<T>(t.p, e, p, push);
+                if (sizeof(T) == 2 && __any_sync(kFull, differ != 0))
+                    exact_params<T>(t, e, h2, s, bc2(ms), [&](int j) {
+                        const int w0 = strip_word(first, 2 * j), w1 = strip_word(first, 2 * j + 1);
+                        return mk2(fminf(2 * j >= left ? old_b : old_a, col_old[w0]), fminf(2 * j + 1 >= left ? old_b : old_a, col_old[w1]));
+                    }, pout);
+                store_params<T>(t.p, e, p, pout, PUSH ? push : nullptr);
                 *reinterpret_cast<uint32_t*>(mc + (e >> 1)) = quantize_m8_safe(m, ms_new, s);
                 *reinterpret_cast<uint32_t*>(vc + (e >> 1)) =
                     pack_u4(cv[1], cv[0], pack_u4(cv[3], cv[2], pack_u4(cv[5], cv[4], pack_u4(cv[7], cv[6], 0u))));
