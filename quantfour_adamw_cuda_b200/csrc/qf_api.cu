@@ -873,12 +873,9 @@ int qf_quantize_block(const float* x, int64_t numel, int map, uint8_t* codes, fl
     const int vec = aligned(x, 16) && aligned(codes, 4);
     const int runs = codec_runs_for(runs_of(numel), 1);
     const unsigned grid = persistent_grid(ceil_div(runs_of(numel), runs), kCodecCtas);
-    if (map)
-        qf::quantize_block_kernel<1><<<grid, qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(x, numel, codes, scales, vec, runs);
-    else
-        qf::quantize_block_kernel<0><<<grid, qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(x, numel, codes, scales, vec, runs);
-    QF_CUDA(cudaGetLastError());
-    return QF_OK;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return map ? launch_chained<qf::quantize_block_kernel<1>>(grid, 0, 0, st, x, numel, codes, scales, vec, runs)
+               : launch_chained<qf::quantize_block_kernel<0>>(grid, 0, 0, st, x, numel, codes, scales, vec, runs);
 }
 
 int qf_dequantize_block(const uint8_t* codes, const float* scales, int64_t numel, int map, float* out, int device,
@@ -894,9 +891,7 @@ int qf_dequantize_block(const uint8_t* codes, const float* scales, int64_t numel
     const int runs = codec_runs_for(runs_of(numel), 4);
     unsigned grid;
     if (int rc = grid_for(ceil_div(runs_of(numel), runs), &grid)) return rc;
-    qf::dequantize_block_kernel<<<grid, qf::kThreads, 0, static_cast<cudaStream_t>(stream)>>>(codes, scales, numel, map, out, vec, runs);
-    QF_CUDA(cudaGetLastError());
-    return QF_OK;
+    return launch_chained<qf::dequantize_block_kernel>(grid, 0, 0, static_cast<cudaStream_t>(stream), codes, scales, numel, map, out, vec, runs);
 }
 
 int qf_quantize_rank1(const float* v, int64_t rows, int64_t cols, uint8_t* codes, float* row_max, float* col_max,
@@ -910,31 +905,30 @@ int qf_quantize_rank1(const float* v, int64_t rows, int64_t cols, uint8_t* codes
         return fail(QF_ERR_BAD_ARG, "qf_quantize_rank1: v / row_max / col_max not 4-byte aligned");
     QF_CUDA(cudaSetDevice(device));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    QF_CUDA(cudaMemsetAsync(row_max, 0, sizeof(float) * rows, st));
-    QF_CUDA(cudaMemsetAsync(col_max, 0, sizeof(float) * cols, st));
+    const unsigned clear_grid = static_cast<unsigned>(std::min<int64_t>(ceil_div(rows + cols, qf::kThreads), sm_count() * 8));
+    if (int rc = launch_chained<qf::rank1_clear_kernel>(clear_grid, 0, 0, st, row_max, static_cast<int>(rows), col_max, static_cast<int>(cols))) return rc;
     const int vec = aligned(v, 16) && aligned(codes, 4);
     const int r = static_cast<int>(rows), c = static_cast<int>(cols);
     if (vec && cols % qf::kPanelCols == 0 && aligned(col_max, 16)) {
         const int64_t panels = cols / qf::kPanelCols;
-        const int max_rows = pre_rows_for(rows * panels), item_rows = codec_runs_for(rows * panels, 1);
+        const int max_rows = pre_rows_for(rows * panels), item_rows = codec_runs_for(rows * panels, 4);
         const int64_t max_items = ceil_div(rows, static_cast<int64_t>(max_rows) * qf::kWarpsPerCta) * panels;
         if (max_items > INT32_MAX) return fail(QF_ERR_BAD_ARG, "too many work items for one launch (%lld)", (long long)max_items);
-        qf::rank1_max_panel_kernel<<<static_cast<unsigned>(max_items), qf::kThreads, 0, st>>>(v, r, c, row_max, col_max, max_rows);
-        qf::rank1_quant_panel_kernel<<<persistent_grid(ceil_div(rows, item_rows) * panels, kCodecCtas), qf::kThreads, 0, st>>>(
-            v, codes, row_max, col_max, r, c, item_rows);
+        if (int rc = launch_chained<qf::rank1_max_panel_kernel>(static_cast<unsigned>(max_items), 0, 0, st, v, r, c, row_max, col_max, max_rows)) return rc;
+        return launch_chained<qf::rank1_quant_panel_kernel>(persistent_grid(ceil_div(rows, item_rows) * panels, kCodecCtas), 0, 0, st, v, codes,
+                                                            row_max, col_max, r, c, item_rows);
     } else if (strip_fits(cols, vec)) {
         const int runs = codec_strip_runs_for(numel);
         const unsigned grid = static_cast<unsigned>(ceil_div(numel, qf::strip_entries(runs)));   // at most 2^62 / 2^13, and memory ends far below 2^43
-        qf::rank1_max_strip_kernel<<<grid, qf::kThreads, qf::strip_dyn_smem() / 2, st>>>(v, r, c, row_max, col_max, runs);
-        qf::rank1_codec_strip_kernel<true><<<grid, qf::kThreads, qf::strip_dyn_smem() / 2, st>>>(v, codes, row_max, col_max, r, c, nullptr, runs);
+        constexpr int smem = qf::strip_dyn_smem() / 2;   // one array of column scalars
+        if (int rc = launch_chained<qf::rank1_max_strip_kernel>(grid, smem, smem, st, v, r, c, row_max, col_max, runs)) return rc;
+        return launch_chained<qf::rank1_codec_strip_kernel<true>>(grid, smem, smem, st, v, codes, row_max, col_max, r, c, nullptr, runs);
     } else {
         unsigned grid;
         if (int rc = grid_for(flat_items(numel), &grid)) return rc;
-        qf::rank1_max_kernel<<<grid, qf::kThreads, 0, st>>>(v, r, c, row_max, col_max);
-        qf::rank1_codec_kernel<true><<<grid, qf::kThreads, 0, st>>>(v, codes, row_max, col_max, r, c, nullptr, vec);
+        if (int rc = launch_chained<qf::rank1_max_kernel>(grid, 0, 0, st, v, r, c, row_max, col_max)) return rc;
+        return launch_chained<qf::rank1_codec_kernel<true>>(grid, 0, 0, st, v, codes, row_max, col_max, r, c, nullptr, vec);
     }
-    QF_CUDA(cudaGetLastError());
-    return QF_OK;
 }
 
 int qf_dequantize_rank1(const uint8_t* codes, const float* row_max, const float* col_max, int64_t rows, int64_t cols,
@@ -952,20 +946,19 @@ int qf_dequantize_rank1(const uint8_t* codes, const float* row_max, const float*
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (vec && cols % qf::kPanelCols == 0 && aligned(col_max, 16)) {
         const int64_t panels = cols / qf::kPanelCols;
-        const int item_rows = codec_runs_for(rows * panels, 1);
-        qf::rank1_dequant_panel_kernel<<<persistent_grid(ceil_div(rows, item_rows) * panels, kCodecCtas), qf::kThreads, 0, st>>>(
-            codes, row_max, col_max, r, c, out, item_rows);
+        const int item_rows = codec_runs_for(rows * panels, 4);
+        return launch_chained<qf::rank1_dequant_panel_kernel>(persistent_grid(ceil_div(rows, item_rows) * panels, kCodecCtas), 0, 0, st, codes,
+                                                              row_max, col_max, r, c, out, item_rows);
     } else if (strip_fits(cols, vec)) {
         const int runs = codec_strip_runs_for(numel);
-        qf::rank1_codec_strip_kernel<false><<<static_cast<unsigned>(ceil_div(numel, qf::strip_entries(runs))), qf::kThreads,
-                                              qf::strip_dyn_smem() / 2, st>>>(nullptr, const_cast<uint8_t*>(codes), row_max, col_max, r, c, out, runs);
+        constexpr int smem = qf::strip_dyn_smem() / 2;
+        return launch_chained<qf::rank1_codec_strip_kernel<false>>(static_cast<unsigned>(ceil_div(numel, qf::strip_entries(runs))), smem, smem, st,
+                                                                   nullptr, const_cast<uint8_t*>(codes), row_max, col_max, r, c, out, runs);
     } else {
         unsigned grid;
         if (int rc = grid_for(flat_items(numel), &grid)) return rc;
-        qf::rank1_codec_kernel<false><<<grid, qf::kThreads, 0, st>>>(nullptr, const_cast<uint8_t*>(codes), row_max, col_max, r, c, out, vec);
+        return launch_chained<qf::rank1_codec_kernel<false>>(grid, 0, 0, st, nullptr, const_cast<uint8_t*>(codes), row_max, col_max, r, c, out, vec);
     }
-    QF_CUDA(cudaGetLastError());
-    return QF_OK;
 }
 
 // ---- the step of one rank-1 tensor for callers that cannot allocate ------------------------------------
