@@ -332,8 +332,9 @@ def single_gpu(args):
                      "traffic_kind": "scaled from an ncu capture of the same kernels on the 355 M-parameter set",
                      "peak_kind": peak_kind, "frac_of_8TBs": achieved / 8000.0,
                      "algorithmic_bytes_per_step": alg_bytes, "kernels_ms": {"pre": pre_ms, "main": main_ms},
-                     "note": "whole step (clear, pre, reciprocals, main panel, main flat, commit: 6 launches) over algorithmic bytes"},
-        "e2e": e2e, "gpu_launches": 6 * args.steps, "clocks": clocks,
+                     "note": "whole step (all launches) over algorithmic bytes"},
+        # roll, first pass, second pass of the matrices, second pass of the vectors
+        "e2e": e2e, "gpu_launches": 4 * args.steps, "clocks": clocks,
     }
     if not args.no_also:
         del opt, params, grads
